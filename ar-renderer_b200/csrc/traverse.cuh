@@ -44,7 +44,7 @@ struct __align__(16) QNode {
     int4 child;  // >= 0: interior QNode; < 0: leaf whose first slot is ~child
     int4 pad;
 };
-// The any-hit traversal addresses the plane vectors by byte offset (slab_nf).
+// The any-hit traversal addresses the plane vectors by byte offset (slab2).
 static_assert(offsetof(QNode, lox) == 0 && offsetof(QNode, loy) == 16 && offsetof(QNode, loz) == 32 &&
                   offsetof(QNode, hix) == 48 && offsetof(QNode, hiy) == 64 && offsetof(QNode, hiz) == 80 &&
                   sizeof(QNode) == 128,
@@ -118,17 +118,60 @@ __device__ __forceinline__ bool box_entry_nb(const TraceRay &r, float lox, float
     return t0 <= t1 && t1 > 0.f;
 }
 
-// box_entry_nb with the near and far planes already chosen by the ray's octant (QNode layout:
-// lo x, y, z at bytes 0, 16, 32, hi at 48, 64, 80): the same products and comparisons, folded
-// with the tMax test; +inf when the box is rejected or entered at or after tMax.
-__device__ __forceinline__ float slab_nf(const TraceRay &r, float nx, float fx, float ny, float fy, float nz, float fz,
-                                         float tMax) {
-    float t0 = fmaxf(fmaxf(__fmul_rn(__fsub_rn(nx, r.o.x), r.inv.x), __fmul_rn(__fsub_rn(ny, r.o.y), r.inv.y)),
-                     __fmul_rn(__fsub_rn(nz, r.o.z), r.inv.z));
-    float t1 = fminf(fminf(__fmul_rn(__fmul_rn(__fsub_rn(fx, r.o.x), r.inv.x), kWiden),
-                           __fmul_rn(__fmul_rn(__fsub_rn(fy, r.o.y), r.inv.y), kWiden)),
-                     __fmul_rn(__fmul_rn(__fsub_rn(fz, r.o.z), r.inv.z), kWiden));
-    return t0 <= t1 && t1 > 0.f && t0 < tMax ? t0 : __int_as_float(0x7f800000);
+// Two floats in one 64-bit register, for the paired FP32 instructions of sm_100 (each half is its own
+// correctly rounded operation, so results are those of the scalar instructions at half the issue slots).
+__device__ __forceinline__ uint64_t pair_of(float lo, float hi) {
+    uint64_t p;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(lo), "f"(hi));
+    return p;
+}
+__device__ __forceinline__ void unpair(uint64_t p, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(p));
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t p;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(p) : "l"(a), "l"(b));
+    return p;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t p;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(p) : "l"(a), "l"(b));
+    return p;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float d;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+
+// box_entry_nb of two boxes at once, with the near and far planes already chosen by the ray's octant
+// (QNode layout: lo x, y, z at bytes 0, 16, 32, hi at 48, 64, 80): the same products and comparisons,
+// folded with the tMax test; +inf when a box is rejected or entered at or after tMax. The exits are
+// widened after their minimum: rounding is monotone, so that is the minimum of the widened exits.
+// A node step is bound by issue slots: pairs, three-operand min / max and one widening a box take about
+// 50 instructions for four boxes instead of 84. Ray-query benchmark (2^24 rays, ms, closest / any hit):
+// 4.25 / 2.96 -> 4.20 / 2.92; 4,096-triangle soup, 2^22 rays: 0.838 / 0.611 -> 0.804 / 0.594.
+__device__ __forceinline__ void slab2(const TraceRay &r, uint64_t nx, uint64_t fx, uint64_t ny, uint64_t fy,
+                                      uint64_t nz, uint64_t fz, float tMax, float &tA, float &tB) {
+    const uint64_t ox = pair_of(-r.o.x, -r.o.x), oy = pair_of(-r.o.y, -r.o.y), oz = pair_of(-r.o.z, -r.o.z);
+    const uint64_t ix = pair_of(r.inv.x, r.inv.x), iy = pair_of(r.inv.y, r.inv.y), iz = pair_of(r.inv.z, r.inv.z);
+    float xa, xb, ya, yb, za, zb;
+    unpair(mul2(add2(nx, ox), ix), xa, xb);
+    unpair(mul2(add2(ny, oy), iy), ya, yb);
+    unpair(mul2(add2(nz, oz), iz), za, zb);
+    const float na = max3(xa, ya, za), nb = max3(xb, yb, zb);
+    unpair(mul2(add2(fx, ox), ix), xa, xb);
+    unpair(mul2(add2(fy, oy), iy), ya, yb);
+    unpair(mul2(add2(fz, oz), iz), za, zb);
+    const float ea = __fmul_rn(min3(xa, ya, za), kWiden), eb = __fmul_rn(min3(xb, yb, zb), kWiden);
+    const float inf = __int_as_float(0x7f800000);
+    tA = na <= ea && ea > 0.f && na < tMax ? na : inf;
+    tB = nb <= eb && eb > 0.f && nb < tMax ? nb : inf;
 }
 
 // Möller-Trumbore in the reference's exact operation order (shape.cpp:202-222).
@@ -444,16 +487,14 @@ __device__ __forceinline__ bool traverse4_step_st(const QNode *__restrict__ node
                 // form that keeps t, u, v live loads all six plane vectors below.
                 const char *nb = reinterpret_cast<const char *>(n);
                 const int ox = r.neg[0] ? 48 : 0, oy = r.neg[1] ? 48 : 0, oz = r.neg[2] ? 48 : 0;
-                const float4 nx = __ldg(reinterpret_cast<const float4 *>(nb + ox));
-                const float4 fx = __ldg(reinterpret_cast<const float4 *>(nb + 48 - ox));
-                const float4 ny = __ldg(reinterpret_cast<const float4 *>(nb + 16 + oy));
-                const float4 fy = __ldg(reinterpret_cast<const float4 *>(nb + 64 - oy));
-                const float4 nz = __ldg(reinterpret_cast<const float4 *>(nb + 32 + oz));
-                const float4 fz = __ldg(reinterpret_cast<const float4 *>(nb + 80 - oz));
-                t0 = slab_nf(r, nx.x, fx.x, ny.x, fy.x, nz.x, fz.x, s.tMax);
-                t1 = slab_nf(r, nx.y, fx.y, ny.y, fy.y, nz.y, fz.y, s.tMax);
-                t2 = slab_nf(r, nx.z, fx.z, ny.z, fy.z, nz.z, fz.z, s.tMax);
-                t3 = slab_nf(r, nx.w, fx.w, ny.w, fy.w, nz.w, fz.w, s.tMax);
+                const ulonglong2 nx = __ldg(reinterpret_cast<const ulonglong2 *>(nb + ox));
+                const ulonglong2 fx = __ldg(reinterpret_cast<const ulonglong2 *>(nb + 48 - ox));
+                const ulonglong2 ny = __ldg(reinterpret_cast<const ulonglong2 *>(nb + 16 + oy));
+                const ulonglong2 fy = __ldg(reinterpret_cast<const ulonglong2 *>(nb + 64 - oy));
+                const ulonglong2 nz = __ldg(reinterpret_cast<const ulonglong2 *>(nb + 32 + oz));
+                const ulonglong2 fz = __ldg(reinterpret_cast<const ulonglong2 *>(nb + 80 - oz));
+                slab2(r, nx.x, fx.x, ny.x, fy.x, nz.x, fz.x, s.tMax, t0, t1);
+                slab2(r, nx.y, fx.y, ny.y, fy.y, nz.y, fz.y, s.tMax, t2, t3);
             } else {
                 const float4 lx = __ldg(&n->lox), ly = __ldg(&n->loy), lz = __ldg(&n->loz);
                 const float4 hx = __ldg(&n->hix), hy = __ldg(&n->hiy), hz = __ldg(&n->hiz);
