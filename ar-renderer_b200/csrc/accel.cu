@@ -16,8 +16,10 @@ namespace prb {
 // busy instead of idling until the warp's longest ray ends. A refill (ray load, reciprocal
 // direction, root-box test, and the finished rays' result stores) runs once kRefillLanes lanes of
 // the warp are idle, or none is busy.
+// kTail (4-wide form): a query with fewer rays than the grid has lanes is spread over the warps, and once
+// the queue has run dry a warp finishes its last rays with all its lanes (traverse4_finish).
 
-template <bool kAny, bool kWide>
+template <bool kAny, bool kWide, bool kTail>
 __global__ void __launch_bounds__(256, 4) k_trace_persist(const void *__restrict__ nodes,
                                                           const LeafPrim *__restrict__ prims, RootInfo root,
                                                           const float4 *__restrict__ rays, int64_t n,
@@ -43,6 +45,9 @@ __global__ void __launch_bounds__(256, 4) k_trace_persist(const void *__restrict
     int64_t idx = 0;
     // pending: this lane's last ray is finished and its result not yet stored.
     bool active = false, exhausted = false, pending = false, overflow = false;
+    const int64_t warps = int64_t(gridDim.x) * (blockDim.x / 32);
+    if (kTail && lane >= (n + warps - 1) / warps) exhausted = true;
+    bool drained = false;
     auto store = [&]() {
         if (kAny) {
             primOut[idx] = s.found ? 1 : 0;
@@ -88,21 +93,34 @@ __global__ void __launch_bounds__(256, 4) k_trace_persist(const void *__restrict
                     pending = !active;
                 }
             }
+            drained = kTail && root.bound <= kCoopBound && __any_sync(full, exhausted);
+            continue;
         }
-        if (__all_sync(full, exhausted)) break;
+        if (!busy) break;
         bool done = false;
-        if (active) {
-            if (kWide)
-                done = traverse4_step_st<kAny, false, false, true>(static_cast<const QNode *>(nodes), prims, r, s, hs,
-                                                                   &overflow);
-            else
-                done = traverse_step<kAny, false>(static_cast<const WNode *>(nodes), prims, r, s, stackRef, stackT,
-                                                  &overflow);
+        if (kWide) {
+            // The queue has run dry and few rays are left: the warp finishes them together, below.
+            if (kTail && drained && coop_ready(busy, active, s.sp)) break;
+            if (leaf_turn(busy, __ballot_sync(full, active && s.ref < 0))) {
+                if (active && s.ref < 0) done = traverse4_leaf<kAny, false, false, true>(prims, r, s, hs);
+            } else if (active && s.ref >= 0) {
+                done = traverse4_node<kAny, true>(static_cast<const QNode *>(nodes), r, s, hs, &overflow);
+            }
+        } else if (active) {
+            done = traverse_step<kAny, false>(static_cast<const WNode *>(nodes), prims, r, s, stackRef, stackT, &overflow);
         }
         if (done) {
             active = false;
             pending = true;
         }
+    }
+    if (kTail) {
+        if (__any_sync(full, active)) {
+            const float tMax = active ? __ldcs(&rays[2 * idx].w) : 0.f;
+            overflow |= traverse4_finish<kAny, false, false, false>(static_cast<const QNode *>(nodes), prims, nullptr,
+                                                                    root.bound, root.ref, r, s, active, hs, tMax);
+        }
+        if (active || pending) store();
     }
     if (overflow) atomicOr(status, 1);
 }
@@ -114,6 +132,12 @@ template <typename K> int resident_blocks(K kernel, int block) {
     return std::max(1, n);
 }
 
+// Up to this many rays the launch's tail, 40 to 80 us with one lane a ray to the end, costs more than
+// the registers that the call of traverse4_finish takes from the loop (7 %). 1M-triangle soup, closest
+// hit, with / without, us: 4,096 rays 84 / 124, 262,144 209 / 241, 1.5M 505 / 526, 4.2M 1153 / 1122,
+// 16.8M 4187 / 3897.
+constexpr int64_t kTailRays = 3 << 20;
+
 // dStatus points at the accel's 16-byte status block: int status at 0, ray counter at 8.
 // wide: the 4-wide tree (fast; hits identical up to the order among exactly equal distances);
 // otherwise the binary tree in the reference's visit order (bvh.cpp:184-190).
@@ -121,35 +145,28 @@ void launch_trace(const DeviceAccel &acc, const prgpu::Ray *dRays, int64_t n, bo
                   float *dT, float *dB1, float *dB2, int *dStatus, cudaStream_t s, int smCount, bool wide) {
     if (n <= 0) return;
     const int block = 256;
-    static int resident[2][2] = {{0, 0}, {0, 0}};
-    if (!resident[0][0]) {
-        resident[0][0] = resident_blocks(k_trace_persist<false, false>, block);
-        resident[0][1] = resident_blocks(k_trace_persist<false, true>, block);
-        resident[1][0] = resident_blocks(k_trace_persist<true, false>, block);
-        resident[1][1] = resident_blocks(k_trace_persist<true, true>, block);
-    }
-    const void *nodes = wide ? acc.qnodes.ptr : acc.nodes.ptr;
-    const int residentAny = resident[1][wide ? 1 : 0], residentClosest = resident[0][wide ? 1 : 0];
+    const auto *r4 = reinterpret_cast<const float4 *>(dRays);
     auto *counter = reinterpret_cast<unsigned long long *>(reinterpret_cast<char *>(dStatus) + 8);
     PRB_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), s));
-    int64_t blocksNeeded = (n + block - 1) / block;
-    const auto *r4 = reinterpret_cast<const float4 *>(dRays);
-    if (anyHit) {
-        int grid = int(std::min<int64_t>(blocksNeeded, int64_t(smCount) * residentAny));
-        if (wide)
-            k_trace_persist<true, true><<<grid, block, 0, s>>>(nodes, acc.prims.as<LeafPrim>(), acc.root, r4, n, dPrim,
-                                                               nullptr, nullptr, nullptr, dStatus, counter);
-        else
-            k_trace_persist<true, false><<<grid, block, 0, s>>>(nodes, acc.prims.as<LeafPrim>(), acc.root, r4, n, dPrim,
-                                                                nullptr, nullptr, nullptr, dStatus, counter);
+    // Blocks needed at one lane a ray, or (tail form) down to one ray a warp.
+    auto launch = [&](auto kernel, int &resident, const void *nodes, int raysPerBlock) {
+        if (!resident) resident = resident_blocks(kernel, block);
+        const int64_t needed = (n + raysPerBlock - 1) / raysPerBlock;
+        const int grid = int(std::min<int64_t>(needed, int64_t(smCount) * resident));
+        kernel<<<grid, block, 0, s>>>(nodes, acc.prims.as<LeafPrim>(), acc.root, r4, n, dPrim, anyHit ? nullptr : dT,
+                                      anyHit ? nullptr : dB1, anyHit ? nullptr : dB2, dStatus, counter);
+    };
+    static int resident[2][3] = {};
+    const void *q = acc.qnodes.ptr, *w = acc.nodes.ptr;
+    if (!wide) {
+        if (anyHit) launch(k_trace_persist<true, false, false>, resident[1][0], w, block);
+        else launch(k_trace_persist<false, false, false>, resident[0][0], w, block);
+    } else if (n <= kTailRays) {
+        if (anyHit) launch(k_trace_persist<true, true, true>, resident[1][1], q, block / 32);
+        else launch(k_trace_persist<false, true, true>, resident[0][1], q, block / 32);
     } else {
-        int grid = int(std::min<int64_t>(blocksNeeded, int64_t(smCount) * residentClosest));
-        if (wide)
-            k_trace_persist<false, true><<<grid, block, 0, s>>>(nodes, acc.prims.as<LeafPrim>(), acc.root, r4, n, dPrim,
-                                                                dT, dB1, dB2, dStatus, counter);
-        else
-            k_trace_persist<false, false><<<grid, block, 0, s>>>(nodes, acc.prims.as<LeafPrim>(), acc.root, r4, n,
-                                                                 dPrim, dT, dB1, dB2, dStatus, counter);
+        if (anyHit) launch(k_trace_persist<true, true, false>, resident[1][2], q, block);
+        else launch(k_trace_persist<false, true, false>, resident[0][2], q, block);
     }
     count_launch();
     PRB_CUDA(cudaGetLastError());

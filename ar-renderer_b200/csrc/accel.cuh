@@ -18,6 +18,7 @@ struct RootInfo {
     float box[6];
     int ref;
     int empty;  // 1 = no nodes: every query misses
+    int bound;  // most entries a depth-first walk of the 4-wide tree holds at a time
 };
 
 struct HostAccel {
@@ -29,7 +30,8 @@ struct HostAccel {
 
 // Collapses the binary tree under interior WNode w into 4-wide nodes: a node takes its two
 // children and, while it has fewer than four, opens the interior child of largest surface area.
-inline int collapse4(const HostAccel &b, int w, std::vector<QNode> *out) {
+// `levels` is raised to the deepest level below `level`.
+inline int collapse4(const HostAccel &b, int w, std::vector<QNode> *out, int level, int *levels) {
     struct Kid {
         int ref;
         float lo[3], hi[3];
@@ -60,6 +62,7 @@ inline int collapse4(const HostAccel &b, int w, std::vector<QNode> *out) {
         kids[best] = two[0];
         kids[nk++] = two[1];
     }
+    *levels = std::max(*levels, level + 1);
     const int idx = int(out->size());
     out->push_back(QNode{});
     float lo[3][4], hi[3][4];
@@ -72,7 +75,7 @@ inline int collapse4(const HostAccel &b, int w, std::vector<QNode> *out) {
         }
         ch[i] = 0;
     }
-    for (int i = 0; i < nk; ++i) ch[i] = kids[i].ref >= 0 ? collapse4(b, kids[i].ref, out) : kids[i].ref;
+    for (int i = 0; i < nk; ++i) ch[i] = kids[i].ref >= 0 ? collapse4(b, kids[i].ref, out, level + 1, levels) : kids[i].ref;
     QNode &q = (*out)[size_t(idx)];
     q.lox = make_float4(lo[0][0], lo[0][1], lo[0][2], lo[0][3]);
     q.loy = make_float4(lo[1][0], lo[1][1], lo[1][2], lo[1][3]);
@@ -212,7 +215,11 @@ bool convert_bvh(const prgpu::BVHNode *nodes, int32_t nodeCount, const int32_t *
     out->qnodes.clear();
     if (out->root.ref >= 0) {
         out->qnodes.reserve(out->nodes.size() / 2 + 1);
-        collapse4(*out, out->root.ref, &out->qnodes);
+        int levels = 0;
+        collapse4(*out, out->root.ref, &out->qnodes, 0, &levels);
+        out->root.bound = 3 * levels + 1;  // a node takes one entry and leaves at most four
+    } else {
+        out->root.bound = 1;
     }
     return true;
 }
@@ -225,7 +232,7 @@ struct DeviceAccel {
     int64_t bytes = 0;
     void upload(const HostAccel &h, cudaStream_t s) {
         size_t nb = std::max<size_t>(1, h.nodes.size()) * sizeof(WNode);
-        size_t pb = std::max<size_t>(1, h.prims.size()) * sizeof(LeafPrim);
+        size_t pb = (h.prims.size() + kLeafPad) * sizeof(LeafPrim);
         nodes.ensure(nb);
         prims.ensure(pb);
         if (!h.nodes.empty())

@@ -174,6 +174,17 @@ __device__ __forceinline__ void slab2(const TraceRay &r, uint64_t nx, uint64_t f
     tB = nb <= eb && eb > 0.f && nb < tMax ? nb : inf;
 }
 
+// slab2 of one box.
+__device__ __forceinline__ float slab_nf(const TraceRay &r, float nx, float fx, float ny, float fy, float nz, float fz,
+                                         float tMax) {
+    const float t0 = max3(__fmul_rn(__fsub_rn(nx, r.o.x), r.inv.x), __fmul_rn(__fsub_rn(ny, r.o.y), r.inv.y),
+                          __fmul_rn(__fsub_rn(nz, r.o.z), r.inv.z));
+    const float t1 = __fmul_rn(min3(__fmul_rn(__fsub_rn(fx, r.o.x), r.inv.x), __fmul_rn(__fsub_rn(fy, r.o.y), r.inv.y),
+                                    __fmul_rn(__fsub_rn(fz, r.o.z), r.inv.z)),
+                               kWiden);
+    return t0 <= t1 && t1 > 0.f && t0 < tMax ? t0 : __int_as_float(0x7f800000);
+}
+
 // Möller-Trumbore in the reference's exact operation order (shape.cpp:202-222).
 __device__ __forceinline__ float dot_rn(float ax, float ay, float az, float bx, float by, float bz) {
     return __fadd_rn(__fadd_rn(__fmul_rn(ax, bx), __fmul_rn(ay, by)), __fmul_rn(az, bz));
@@ -447,6 +458,7 @@ constexpr int kRefillLanes = 8;
 
 template <int kShort, int kThreads>
 struct HybridStack {
+    static constexpr int kRowStride = kThreads;
     int2 *sh;
     int ref[kStackSize - kShort];
     float t[kStackSize - kShort];
@@ -469,113 +481,130 @@ struct HybridStack {
 // same t, u, v bit for bit. Fewer live registers in the loop let the slab planes be selected by
 // address as for any hit (ray-query benchmark, closest hit: 3,821 -> 3,926 Mrays/s; either change
 // alone was slower: 3,730 and 3,667).
-template <bool kAny, bool kSpheres, bool kSkipTransparent = false, bool kDeferUV = false, class Stack>
-__device__ __forceinline__ bool traverse4_step_st(const QNode *__restrict__ nodes, const LeafPrim *__restrict__ prims,
-                                                  const TraceRay &r, TravState &s, Stack &stack, bool *overflow,
-                                                  const uint8_t *__restrict__ cls = nullptr) {
-    if (s.ref >= 0) {
-        const QNode *n = nodes + s.ref;
-        float t0, t1, t2, t3;
-        const float inf = __int_as_float(0x7f800000);
-        int4 ch;
-        if constexpr (kAny || kDeferUV) {
-            ch = __ldg(&n->child);
-            if (!r.infInv) {
-                // The near and far planes chosen by address from the ray's octant (six loads, no
-                // per-child selects). Measured on the ray-query benchmark: any hit 5,314 -> 5,689
-                // Mrays/s; closest hit only together with kDeferUV (see above); the closest-hit
-                // form that keeps t, u, v live loads all six plane vectors below.
-                const char *nb = reinterpret_cast<const char *>(n);
-                const int ox = r.neg[0] ? 48 : 0, oy = r.neg[1] ? 48 : 0, oz = r.neg[2] ? 48 : 0;
-                const ulonglong2 nx = __ldg(reinterpret_cast<const ulonglong2 *>(nb + ox));
-                const ulonglong2 fx = __ldg(reinterpret_cast<const ulonglong2 *>(nb + 48 - ox));
-                const ulonglong2 ny = __ldg(reinterpret_cast<const ulonglong2 *>(nb + 16 + oy));
-                const ulonglong2 fy = __ldg(reinterpret_cast<const ulonglong2 *>(nb + 64 - oy));
-                const ulonglong2 nz = __ldg(reinterpret_cast<const ulonglong2 *>(nb + 32 + oz));
-                const ulonglong2 fz = __ldg(reinterpret_cast<const ulonglong2 *>(nb + 80 - oz));
-                slab2(r, nx.x, fx.x, ny.x, fy.x, nz.x, fz.x, s.tMax, t0, t1);
-                slab2(r, nx.y, fx.y, ny.y, fy.y, nz.y, fz.y, s.tMax, t2, t3);
-            } else {
-                const float4 lx = __ldg(&n->lox), ly = __ldg(&n->loy), lz = __ldg(&n->loz);
-                const float4 hx = __ldg(&n->hix), hy = __ldg(&n->hiy), hz = __ldg(&n->hiz);
-                t0 = box_entry(r, lx.x, ly.x, lz.x, hx.x, hy.x, hz.x, &t0) && t0 < s.tMax ? t0 : inf;
-                t1 = box_entry(r, lx.y, ly.y, lz.y, hx.y, hy.y, hz.y, &t1) && t1 < s.tMax ? t1 : inf;
-                t2 = box_entry(r, lx.z, ly.z, lz.z, hx.z, hy.z, hz.z, &t2) && t2 < s.tMax ? t2 : inf;
-                t3 = box_entry(r, lx.w, ly.w, lz.w, hx.w, hy.w, hz.w, &t3) && t3 < s.tMax ? t3 : inf;
-            }
-        } else {
-            const float4 lx = __ldg(&n->lox), ly = __ldg(&n->loy), lz = __ldg(&n->loz);
-            const float4 hx = __ldg(&n->hix), hy = __ldg(&n->hiy), hz = __ldg(&n->hiz);
-            ch = __ldg(&n->child);
-            if (!r.infInv) {
-                t0 = box_entry_nb(r, lx.x, ly.x, lz.x, hx.x, hy.x, hz.x, &t0) && t0 < s.tMax ? t0 : inf;
-                t1 = box_entry_nb(r, lx.y, ly.y, lz.y, hx.y, hy.y, hz.y, &t1) && t1 < s.tMax ? t1 : inf;
-                t2 = box_entry_nb(r, lx.z, ly.z, lz.z, hx.z, hy.z, hz.z, &t2) && t2 < s.tMax ? t2 : inf;
-                t3 = box_entry_nb(r, lx.w, ly.w, lz.w, hx.w, hy.w, hz.w, &t3) && t3 < s.tMax ? t3 : inf;
-            } else {
-                t0 = box_entry(r, lx.x, ly.x, lz.x, hx.x, hy.x, hz.x, &t0) && t0 < s.tMax ? t0 : inf;
-                t1 = box_entry(r, lx.y, ly.y, lz.y, hx.y, hy.y, hz.y, &t1) && t1 < s.tMax ? t1 : inf;
-                t2 = box_entry(r, lx.z, ly.z, lz.z, hx.z, hy.z, hz.z, &t2) && t2 < s.tMax ? t2 : inf;
-                t3 = box_entry(r, lx.w, ly.w, lz.w, hx.w, hy.w, hz.w, &t3) && t3 < s.tMax ? t3 : inf;
-            }
-        }
-        int r0 = ch.x, r1 = ch.y, r2 = ch.z, r3 = ch.w;
-        // Sorting network for 4 (5 compare-exchanges); misses sort last at +inf.
-        cswap(t0, r0, t1, r1);
-        cswap(t2, r2, t3, r3);
-        cswap(t0, r0, t2, r2);
-        cswap(t1, r1, t3, r3);
-        cswap(t1, r1, t2, r2);
-        if (t0 < inf) {
-            const int extra = (t1 < inf) + (t2 < inf) + (t3 < inf);
-            if (s.sp + extra > kStackSize) {
-                *overflow = true;
-                return true;
-            }
-            if (t3 < inf) stack.put(s.sp++, r3, t3);
-            if (t2 < inf) stack.put(s.sp++, r2, t2);
-            if (t1 < inf) stack.put(s.sp++, r1, t1);
-            s.ref = r0;
-            return false;
-        }
-    } else {
-        const LeafPrim *p = prims + ~s.ref;
-        for (bool last = false; !last; ++p) {
-            float4 v0 = __ldg(&p->v0), v1 = __ldg(&p->v1), v2 = __ldg(&p->v2);
-            last = __float_as_int(v2.w) != 0;
-            float t, u = 0.f, v = 0.f;
-            bool h;
-            if (kSpheres && __float_as_int(v1.w) == 1)
-                h = hit_sphere(r, v0, v1, s.tMax, &t);
-            else
-                h = hit_triangle(r, v0, v1, v2, s.tMax, &t, &u, &v);
-            if (h) {
-                if (kSkipTransparent && (__ldg(cls + __float_as_int(v0.w)) & kTransparentBit)) {
-                    s.crossed = true;
-                    continue;
-                }
-                s.found = true;
-                if (kAny) return true;
-                s.tMax = t;
-                if constexpr (kDeferUV) {
-                    s.hit.prim = int(p - prims);
-                } else {
-                    s.hit.t = t;
-                    s.hit.u = u;
-                    s.hit.v = v;
-                    s.hit.prim = __float_as_int(v0.w);
-                }
-            }
-        }
-    }
+// Takes the next deferred child whose entry is still before tMax; false: the traversal is finished.
+template <class Stack> __device__ __forceinline__ bool traverse4_pop(TravState &s, Stack &stack) {
     while (s.sp > 0) {
         --s.sp;
         if (stack.dist(s.sp) < s.tMax) {
             s.ref = stack.node(s.sp);
-            return false;
+            return true;
         }
     }
-    return true;
+    return false;
+}
+
+// One interior node (s.ref >= 0). Returns true when the ray's traversal is finished.
+template <bool kAny, bool kDeferUV, class Stack>
+__device__ __forceinline__ bool traverse4_node(const QNode *__restrict__ nodes, const TraceRay &r, TravState &s,
+                                               Stack &stack, bool *overflow) {
+    const QNode *n = nodes + s.ref;
+    float t0, t1, t2, t3;
+    const float inf = __int_as_float(0x7f800000);
+    int4 ch;
+    if constexpr (kAny || kDeferUV) {
+        ch = __ldg(&n->child);
+        if (!r.infInv) {
+            // The near and far planes chosen by address from the ray's octant (six loads, no
+            // per-child selects). Measured on the ray-query benchmark: any hit 5,314 -> 5,689
+            // Mrays/s; closest hit only together with kDeferUV (see above); the closest-hit
+            // form that keeps t, u, v live loads all six plane vectors below.
+            const char *nb = reinterpret_cast<const char *>(n);
+            const int ox = r.neg[0] ? 48 : 0, oy = r.neg[1] ? 48 : 0, oz = r.neg[2] ? 48 : 0;
+            const ulonglong2 nx = __ldg(reinterpret_cast<const ulonglong2 *>(nb + ox));
+            const ulonglong2 fx = __ldg(reinterpret_cast<const ulonglong2 *>(nb + 48 - ox));
+            const ulonglong2 ny = __ldg(reinterpret_cast<const ulonglong2 *>(nb + 16 + oy));
+            const ulonglong2 fy = __ldg(reinterpret_cast<const ulonglong2 *>(nb + 64 - oy));
+            const ulonglong2 nz = __ldg(reinterpret_cast<const ulonglong2 *>(nb + 32 + oz));
+            const ulonglong2 fz = __ldg(reinterpret_cast<const ulonglong2 *>(nb + 80 - oz));
+            slab2(r, nx.x, fx.x, ny.x, fy.x, nz.x, fz.x, s.tMax, t0, t1);
+            slab2(r, nx.y, fx.y, ny.y, fy.y, nz.y, fz.y, s.tMax, t2, t3);
+        } else {
+            const float4 lx = __ldg(&n->lox), ly = __ldg(&n->loy), lz = __ldg(&n->loz);
+            const float4 hx = __ldg(&n->hix), hy = __ldg(&n->hiy), hz = __ldg(&n->hiz);
+            t0 = box_entry(r, lx.x, ly.x, lz.x, hx.x, hy.x, hz.x, &t0) && t0 < s.tMax ? t0 : inf;
+            t1 = box_entry(r, lx.y, ly.y, lz.y, hx.y, hy.y, hz.y, &t1) && t1 < s.tMax ? t1 : inf;
+            t2 = box_entry(r, lx.z, ly.z, lz.z, hx.z, hy.z, hz.z, &t2) && t2 < s.tMax ? t2 : inf;
+            t3 = box_entry(r, lx.w, ly.w, lz.w, hx.w, hy.w, hz.w, &t3) && t3 < s.tMax ? t3 : inf;
+        }
+    } else {
+        const float4 lx = __ldg(&n->lox), ly = __ldg(&n->loy), lz = __ldg(&n->loz);
+        const float4 hx = __ldg(&n->hix), hy = __ldg(&n->hiy), hz = __ldg(&n->hiz);
+        ch = __ldg(&n->child);
+        if (!r.infInv) {
+            t0 = box_entry_nb(r, lx.x, ly.x, lz.x, hx.x, hy.x, hz.x, &t0) && t0 < s.tMax ? t0 : inf;
+            t1 = box_entry_nb(r, lx.y, ly.y, lz.y, hx.y, hy.y, hz.y, &t1) && t1 < s.tMax ? t1 : inf;
+            t2 = box_entry_nb(r, lx.z, ly.z, lz.z, hx.z, hy.z, hz.z, &t2) && t2 < s.tMax ? t2 : inf;
+            t3 = box_entry_nb(r, lx.w, ly.w, lz.w, hx.w, hy.w, hz.w, &t3) && t3 < s.tMax ? t3 : inf;
+        } else {
+            t0 = box_entry(r, lx.x, ly.x, lz.x, hx.x, hy.x, hz.x, &t0) && t0 < s.tMax ? t0 : inf;
+            t1 = box_entry(r, lx.y, ly.y, lz.y, hx.y, hy.y, hz.y, &t1) && t1 < s.tMax ? t1 : inf;
+            t2 = box_entry(r, lx.z, ly.z, lz.z, hx.z, hy.z, hz.z, &t2) && t2 < s.tMax ? t2 : inf;
+            t3 = box_entry(r, lx.w, ly.w, lz.w, hx.w, hy.w, hz.w, &t3) && t3 < s.tMax ? t3 : inf;
+        }
+    }
+    int r0 = ch.x, r1 = ch.y, r2 = ch.z, r3 = ch.w;
+    // Sorting network for 4 (5 compare-exchanges); misses sort last at +inf.
+    cswap(t0, r0, t1, r1);
+    cswap(t2, r2, t3, r3);
+    cswap(t0, r0, t2, r2);
+    cswap(t1, r1, t3, r3);
+    cswap(t1, r1, t2, r2);
+    if (t0 < inf) {
+        const int extra = (t1 < inf) + (t2 < inf) + (t3 < inf);
+        if (s.sp + extra > kStackSize) {
+            *overflow = true;
+            return true;
+        }
+        if (t3 < inf) stack.put(s.sp++, r3, t3);
+        if (t2 < inf) stack.put(s.sp++, r2, t2);
+        if (t1 < inf) stack.put(s.sp++, r1, t1);
+        s.ref = r0;
+        return false;
+    }
+    return !traverse4_pop(s, stack);
+}
+
+// One leaf (s.ref < 0). Returns true when the ray's traversal is finished.
+template <bool kAny, bool kSpheres, bool kSkipTransparent, bool kDeferUV, class Stack>
+__device__ __forceinline__ bool traverse4_leaf(const LeafPrim *__restrict__ prims, const TraceRay &r, TravState &s,
+                                               Stack &stack, const uint8_t *__restrict__ cls = nullptr) {
+    const LeafPrim *p = prims + ~s.ref;
+    for (bool last = false; !last; ++p) {
+        float4 v0 = __ldg(&p->v0), v1 = __ldg(&p->v1), v2 = __ldg(&p->v2);
+        last = __float_as_int(v2.w) != 0;
+        float t, u = 0.f, v = 0.f;
+        bool h;
+        if (kSpheres && __float_as_int(v1.w) == 1)
+            h = hit_sphere(r, v0, v1, s.tMax, &t);
+        else
+            h = hit_triangle(r, v0, v1, v2, s.tMax, &t, &u, &v);
+        if (h) {
+            if (kSkipTransparent && (__ldg(cls + __float_as_int(v0.w)) & kTransparentBit)) {
+                s.crossed = true;
+                continue;
+            }
+            s.found = true;
+            if (kAny) return true;
+            s.tMax = t;
+            if constexpr (kDeferUV) {
+                s.hit.prim = int(p - prims);
+            } else {
+                s.hit.t = t;
+                s.hit.u = u;
+                s.hit.v = v;
+                s.hit.prim = __float_as_int(v0.w);
+            }
+        }
+    }
+    return !traverse4_pop(s, stack);
+}
+
+template <bool kAny, bool kSpheres, bool kSkipTransparent = false, bool kDeferUV = false, class Stack>
+__device__ __forceinline__ bool traverse4_step_st(const QNode *__restrict__ nodes, const LeafPrim *__restrict__ prims,
+                                                  const TraceRay &r, TravState &s, Stack &stack, bool *overflow,
+                                                  const uint8_t *__restrict__ cls = nullptr) {
+    if (s.ref >= 0) return traverse4_node<kAny, kDeferUV>(nodes, r, s, stack, overflow);
+    return traverse4_leaf<kAny, kSpheres, kSkipTransparent, kDeferUV>(prims, r, s, stack, cls);
 }
 
 // The hit of a kDeferUV traversal: the winning leaf slot's test repeated (no tMax bound), which
@@ -595,12 +624,268 @@ __device__ __forceinline__ Hit finish_hit(const LeafPrim *__restrict__ prims, co
     return h;
 }
 
+// Cooperative form of the 4-wide traversal: a warp finishes the at most eight rays its lanes still
+// hold. The time of a query is at least that of its longest ray, and one lane takes a step per node or
+// leaf, each a dependent load and a chain of arithmetic: on the benchmark soups a launch of a few
+// thousand rays took 70 to 110 us, and every larger launch ended in such a tail. Here groups of four
+// lanes take entries off the rays' stacks (one entry per ray and step with more than four rays left, up
+// to eight with one), each lane tests one child box or one of a leaf's triangles, and what is hit goes
+// back on the stack, so a ray takes a step per level of the tree rather than per node. Measured (B200,
+// closest hit, us, one lane a ray to the end / this): 1,000 rays, 4,096 triangles 81 / 32; 4,096 rays,
+// 100,003 triangles 112 / 56; 1.5M rays, 100,003 triangles 450 / 421.
+// Box and triangle arithmetic are those of the other traversals and a deferred entry is dropped under
+// the same condition, so hits agree up to the order among exactly equal distances. An accepted distance
+// that is not a number (a determinant whose reciprocal overflows) makes the outcome depend on the visit
+// order: such a ray is handed back (true in its lane) for the one-lane traversal to start over.
+//
+// The rays' own lanes keep r and st; stacks move in place from the lanes' columns to regions of 64
+// entries (4 columns of the warp's 32, entry e in row e / 4). `bound` is the most entries a depth-first
+// walk of the tree holds at a time; a step takes more than one entry of a ray only while its region
+// then still has room for such a walk, so a region cannot overflow.
+constexpr int kCoopRays = 8, kRayLanes = 4;
+constexpr int kLeafPad = kRayLanes - 1;  // records past the leaf array that the lanes of a group may load
+constexpr int kCoopBound = kStackSize - 24;  // trees with a larger bound are left to the one-lane traversal
+
+struct CoopState {
+    TravState s;
+    bool redo;
+};
+
+// Out of line: inlined into the persistent kernels it cost their loops registers (closest hits of the
+// 2^24-ray benchmark 4.20 -> 4.71 ms). Hence only rays whose stack is within the shared columns.
+template <bool kAny, bool kSpheres, bool kSkipTransparent, bool kBatch, int kRow>
+__device__ __noinline__ CoopState traverse4_coop(const QNode *nodes, const LeafPrim *prims, const uint8_t *cls,
+                                                 int bound, V3 o, V3 d, TravState st, bool active, int2 *column) {
+    static_assert(kShortStack * 32 == kCoopRays * kStackSize, "the regions fill the warp's columns");
+    __builtin_assume(__isShared(column));
+    const unsigned full = 0xffffffffu;
+    const float inf = __int_as_float(0x7f800000);
+    const int lane = threadIdx.x & 31, sub = lane & (kRayLanes - 1), group = lane / kRayLanes;
+    int2 *warpStack = column - lane;  // column 0 of this warp
+    const TraceRay r = make_trace_ray(o, d);
+    unsigned rays = __ballot_sync(full, active);
+    const int region = __popc(rays & ((1u << lane) - 1u));
+    // In place: row e is read by every ray before entry e lands in row e / 4.
+    for (int e = 0; __any_sync(full, active && e < st.sp); ++e) {
+        int2 v = make_int2(0, 0);
+        if (active && e < st.sp) v = column[e * kRow];
+        __syncwarp();
+        if (active && e < st.sp) warpStack[(e >> 2) * kRow + 4 * region + (e & 3)] = v;
+        __syncwarp();
+    }
+    if (active) {
+        warpStack[(st.sp >> 2) * kRow + 4 * region + (st.sp & 3)] = make_int2(st.ref, __float_as_int(-inf));
+        ++st.sp;
+    }
+    __syncwarp();
+    bool redo = false;
+    unsigned assigned = 0;
+    // The ray this lane works for: its own lane, its region, its data.
+    int home = 0, myRegion = 0, perRay = 1;
+    bool mine = false;
+    TraceRay q = r;
+    while (rays) {
+        if (rays != assigned) {
+            assigned = rays;
+            const int m = __popc(rays);
+            perRay = m > 4 ? 1 : (m > 2 ? 2 : (m > 1 ? 4 : 8));
+            const int i = group / perRay;
+            mine = i < m;
+            unsigned left = rays;
+            for (int k = 0; k < i; ++k) left &= left - 1u;
+            home = mine ? __ffs(left) - 1 : 0;
+            myRegion = __shfl_sync(full, region, home);
+            q.o = {__shfl_sync(full, r.o.x, home), __shfl_sync(full, r.o.y, home), __shfl_sync(full, r.o.z, home)};
+            q.d = {__shfl_sync(full, r.d.x, home), __shfl_sync(full, r.d.y, home), __shfl_sync(full, r.d.z, home)};
+            q.inv = {__shfl_sync(full, r.inv.x, home), __shfl_sync(full, r.inv.y, home),
+                     __shfl_sync(full, r.inv.z, home)};
+            q.neg[0] = q.inv.x < 0.f;
+            q.neg[1] = q.inv.y < 0.f;
+            q.neg[2] = q.inv.z < 0.f;
+            q.infInv = isinf(q.inv.x) || isinf(q.inv.y) || isinf(q.inv.z);
+        }
+        const QNode *qn = nodes;
+        const LeafPrim *lp = prims;
+        const uint8_t *pc = cls;
+        int qb = bound;
+        if (kBatch) {
+            qn = reinterpret_cast<const QNode *>(__shfl_sync(full, reinterpret_cast<unsigned long long>(nodes), home));
+            lp = reinterpret_cast<const LeafPrim *>(__shfl_sync(full, reinterpret_cast<unsigned long long>(prims), home));
+            if (kSkipTransparent)
+                pc = reinterpret_cast<const uint8_t *>(__shfl_sync(full, reinterpret_cast<unsigned long long>(cls), home));
+            qb = __shfl_sync(full, bound, home);
+        }
+        int sp = __shfl_sync(full, st.sp, home);
+        float tMax = __shfl_sync(full, st.tMax, home);
+        const int take = min(min(perRay, sp), max(1, (kStackSize - qb - sp) / 3));
+        const int turn = group & (perRay - 1);  // 0 takes the topmost entry
+        int2 *reg = warpStack + 4 * myRegion;
+        int ref = 0;
+        bool work = mine && turn < take;
+        if (work) {
+            const int e = sp - 1 - turn;
+            const int2 v = reg[(e >> 2) * kRow + (e & 3)];
+            ref = v.x;
+            work = __int_as_float(v.y) < tMax;
+        }
+        __syncwarp();
+        float t = inf;   // entry distance of the child, or the leaf's own for its next four triangles
+        int next = 0;
+        bool hit = false, last = false, nan = false, wall = false;
+        float th = inf;
+        if (work) {
+            if (ref >= 0) {
+                const char *nb = reinterpret_cast<const char *>(qn + ref) + 4 * sub;
+                const int ox = q.neg[0] ? 48 : 0, oy = q.neg[1] ? 48 : 0, oz = q.neg[2] ? 48 : 0;
+                const float nx = __ldg(reinterpret_cast<const float *>(nb + ox));
+                const float fx = __ldg(reinterpret_cast<const float *>(nb + 48 - ox));
+                const float ny = __ldg(reinterpret_cast<const float *>(nb + 16 + oy));
+                const float fy = __ldg(reinterpret_cast<const float *>(nb + 64 - oy));
+                const float nz = __ldg(reinterpret_cast<const float *>(nb + 32 + oz));
+                const float fz = __ldg(reinterpret_cast<const float *>(nb + 80 - oz));
+                next = __ldg(reinterpret_cast<const int *>(nb + 96));
+                if (!q.infInv) {
+                    t = slab_nf(q, nx, fx, ny, fy, nz, fz, tMax);
+                } else {
+                    const bool bx = q.neg[0], by = q.neg[1], bz = q.neg[2];
+                    float te;
+                    t = box_entry(q, bx ? fx : nx, by ? fy : ny, bz ? fz : nz, bx ? nx : fx, by ? ny : fy, bz ? nz : fz,
+                                  &te) && te < tMax ? te : inf;
+                }
+            } else {
+                // Slots past the leaf's last belong to other leaves or are padding: loaded, not tested.
+                const LeafPrim *p = lp + ~ref + sub;
+                const float4 v0 = __ldg(&p->v0), v1 = __ldg(&p->v1), v2 = __ldg(&p->v2);
+                last = __float_as_int(v2.w) != 0;
+                const unsigned quad = 0xfu << (lane & ~3);
+                const unsigned ends = (__ballot_sync(quad, last) >> (lane & ~3)) & 0xfu;
+                if (ends == 0u || sub < __ffs(ends)) {
+                    float u, v;
+                    if (kSpheres && __float_as_int(v1.w) == 1)
+                        hit = hit_sphere(q, v0, v1, tMax, &th);
+                    else
+                        hit = hit_triangle(q, v0, v1, v2, tMax, &th, &u, &v);
+                    if (kSkipTransparent && hit && (__ldg(pc + __float_as_int(v0.w)) & kTransparentBit)) {
+                        wall = true;
+                        hit = false;
+                    }
+                    nan = hit && !(th == th);
+                }
+                if (ends == 0u && sub == 0) {
+                    t = -inf;
+                    next = ref - kRayLanes;  // ~(slot + 4)
+                }
+            }
+        }
+        __syncwarp();
+        const unsigned lanesOfRay = (perRay == 8 ? full : (1u << (kRayLanes * perRay)) - 1u)
+                                    << (lane & ~(kRayLanes * perRay - 1));
+        const int myFirst = __popc(rays & ((1u << lane) - 1u)) * kRayLanes * perRay;  // of the ray this lane owns
+        const bool own = (rays >> lane) & 1u;
+        const unsigned ownLanes = own ? (perRay == 8 ? full : (1u << (kRayLanes * perRay)) - 1u) << myFirst : 0u;
+        const unsigned hits = __ballot_sync(full, hit);
+        if (hits) {
+            if (!kAny) {
+                float best = hit ? th : inf;
+                for (int k = 1; k < kRayLanes * perRay; k <<= 1) best = fminf(best, __shfl_xor_sync(full, best, k));
+                const unsigned win = __ballot_sync(full, hit && th == best);
+                const unsigned w = win & ownLanes;
+                const int src = w ? __ffs(w) - 1 : 0;
+                const float tb = __shfl_sync(full, th, src);
+                const int rb = __shfl_sync(full, ref, src);
+                if (w) {
+                    st.tMax = tb;
+                    st.hit.prim = ~rb + (src & (kRayLanes - 1));
+                }
+                tMax = best < tMax ? best : tMax;
+                if (!(t < tMax)) t = inf;
+            }
+            if (hits & ownLanes) st.found = true;
+            if (__ballot_sync(full, nan) & ownLanes) redo = true;
+        }
+        if (kSkipTransparent && (__ballot_sync(full, wall) & ownLanes)) st.crossed = true;
+        // Push: the later turns' children below the earlier ones', within a group farthest first.
+        int rank = 0;
+#pragma unroll
+        for (int k = 1; k < kRayLanes; ++k) {
+            const float o = __shfl_xor_sync(full, t, k);
+            rank += o < t || (o == t && (sub ^ k) < sub);
+        }
+        const unsigned push = __ballot_sync(full, t < inf);
+        if (t < inf) {
+            const unsigned mask = push & lanesOfRay;
+            const int below = __popc(mask & ~((2u << (lane | 3)) - 1u));
+            const int inGroup = __popc(mask & (0xfu << (lane & ~3)));
+            const int e = sp - take + below + inGroup - 1 - rank;
+            reg[(e >> 2) * kRow + (e & 3)] = make_int2(next, __float_as_int(t));
+        }
+        if (own) {
+            const int b = kBatch ? bound : qb;
+            const int took = min(min(perRay, st.sp), max(1, (kStackSize - b - st.sp) / 3));
+            st.sp += __popc(push & ownLanes) - took;
+        }
+        __syncwarp();
+        rays = __ballot_sync(full, own && st.sp > 0 && !redo && !(kAny && st.found));
+    }
+    return CoopState{st, redo};
+}
+
 template <bool kAny, bool kSpheres, bool kSkipTransparent = false>
 __device__ __forceinline__ bool traverse4_step(const QNode *__restrict__ nodes, const LeafPrim *__restrict__ prims,
                                                const TraceRay &r, TravState &s, int *stackRef, float *stackT,
                                                bool *overflow, const uint8_t *__restrict__ cls = nullptr) {
     LocalStack st{stackRef, stackT};
     return traverse4_step_st<kAny, kSpheres, kSkipTransparent>(nodes, prims, r, s, st, overflow, cls);
+}
+
+// A whole depth-first traversal by one lane, for the rare ray that traverse4_coop hands back. Out of
+// line, with its own copies, so that the kernels' loops keep their registers.
+template <bool kAny, bool kSpheres, bool kSkipTransparent>
+__device__ __noinline__ TravState traverse4_alone(const QNode *nodes, const LeafPrim *prims, const uint8_t *cls,
+                                                  int rootRef, V3 o, V3 d, float tMax, bool *overflow) {
+    int stackRef[kStackSize];
+    float stackT[kStackSize];
+    LocalStack stack{stackRef, stackT};
+    const TraceRay r = make_trace_ray(o, d);
+    TravState s{};
+    s.ref = rootRef;
+    s.tMax = tMax;
+    s.hit.prim = -1;
+    while (!traverse4_step_st<kAny, kSpheres, kSkipTransparent, true>(nodes, prims, r, s, stack, overflow, cls)) {
+    }
+    return s;
+}
+
+// Whether a warp whose queue has run dry should stop its loop and finish its rays (busy: the lanes that
+// hold one) with traverse4_finish: few enough rays, their stacks within shared memory. The caller has
+// checked the tree's bound.
+__device__ __forceinline__ bool coop_ready(unsigned busy, bool active, int sp) {
+    return __popc(busy) <= kCoopRays && __all_sync(0xffffffffu, !active || sp <= kShortStack);
+}
+
+// A warp's step is either a node for the lanes at a node or a leaf for those at a leaf: with both in
+// every step, the leaf code ran with two or three lanes. Lanes at a leaf wait until kLeafLanes do, or
+// until no lane is at a node. Ray-query benchmark (2^24 rays, closest /
+// any hit, ms): both in every step 4.20 / 2.92; from 6 lanes 3.96 / 2.77, 8 lanes 3.90 / 2.74; 12 and 16
+// were 1 and 5 % slower than 8.
+constexpr int kLeafLanes = 8;
+__device__ __forceinline__ bool leaf_turn(unsigned busy, unsigned leaves) {
+    return __popc(leaves) >= kLeafLanes || leaves == busy;
+}
+
+// The end of a persistent traversal kernel: the warp's last rays (lanes with active) traced to their
+// end, `tMax` being what each began with. Returns true when a one-lane traversal ran out of stack.
+template <bool kAny, bool kSpheres, bool kSkipTransparent, bool kBatch, class Stack>
+__device__ __forceinline__ bool traverse4_finish(const QNode *nodes, const LeafPrim *prims, const uint8_t *cls,
+                                                 int bound, int rootRef, const TraceRay &r, TravState &st, bool active,
+                                                 Stack &stack, float tMax) {
+    bool overflow = false;
+    const CoopState c = traverse4_coop<kAny, kSpheres, kSkipTransparent, kBatch, Stack::kRowStride>(
+        nodes, prims, cls, bound, r.o, r.d, st, active, stack.sh);
+    st = c.s;
+    if (c.redo)
+        st = traverse4_alone<kAny, kSpheres, kSkipTransparent>(nodes, prims, cls, rootRef, r.o, r.d, tMax, &overflow);
+    return overflow;
 }
 
 } // namespace prb

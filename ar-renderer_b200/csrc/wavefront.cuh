@@ -1209,8 +1209,13 @@ __global__ void __launch_bounds__(256, kSpheres ? 1 : 4) k_extend(DevScene s0, c
     int j = 0;
     const QNode *nodes = s0.qnodes;
     const LeafPrim *leaves = s0.leaves;
-    bool active = false, exhausted = n == 0, pending = false, overflow = false;
-    while (!__all_sync(full, exhausted)) {
+    bool active = false, pending = false, overflow = false;
+    // A queue shorter than the lanes of the grid is spread over the warps.
+    const int warps = gridDim.x * (256 / 32);
+    bool exhausted = lane >= (n + warps - 1) / warps;
+    bool drained = false;
+    int bound = s0.root.bound, rootRef = s0.root.ref;
+    while (true) {
         const bool idle = !active && !exhausted;
         const unsigned need = __ballot_sync(full, idle), busy = __ballot_sync(full, active);
         if (need && (__popc(need) >= kRefillLanes || !busy)) {
@@ -1243,15 +1248,37 @@ __global__ void __launch_bounds__(256, kSpheres ? 1 : 4) k_extend(DevScene s0, c
                                        s.root.box[5], &te) &&
                              te < kInf;
                     st.ref = s.root.ref;
+                    if (kBatch) {
+                        bound = s.root.bound;
+                        rootRef = s.root.ref;
+                    }
                     // A ray that misses the root: a miss (t, u, v 0), stored at the next refill.
                     pending = !active;
                 }
             }
+            drained = __any_sync(full, exhausted) && __all_sync(full, !active || bound <= kCoopBound);
+            continue;
         }
-        if (active && traverse4_step_st<false, kSpheres, false, true>(nodes, leaves, r, st, hs, &overflow)) {
+        if (!busy) break;
+        // The queue has run dry and few rays are left: the warp finishes them together, below.
+        if (drained && coop_ready(busy, active, st.sp)) break;
+        bool done = false;
+        if (leaf_turn(busy, __ballot_sync(full, active && st.ref < 0))) {
+            if (active && st.ref < 0) done = traverse4_leaf<false, kSpheres, false, true>(leaves, r, st, hs);
+        } else if (active && st.ref >= 0) {
+            done = traverse4_node<false, true>(nodes, r, st, hs, &overflow);
+        }
+        if (done) {
             active = false;
             pending = true;
         }
+    }
+    if (__any_sync(full, active))
+        overflow |= traverse4_finish<false, kSpheres, false, kBatch>(nodes, leaves, nullptr, bound, rootRef, r, st, active,
+                                                                     hs, kInf);
+    if (active || pending) {
+        const Hit h = finish_hit<kSpheres>(leaves, r, st);
+        P.hit[j] = make_float4(h.t, h.u, h.v, __int_as_float(h.prim));
     }
     if (overflow) atomicOr(counters + kCntStatus, kStatusStack);
 }
@@ -1752,27 +1779,35 @@ __global__ void __launch_bounds__(256, (kSpheres || kMedia || kWalls) ? 1 : 4)
     const uint8_t *cls = s0.primClass;
     // pending: this lane's segment is traced and its outcome (accept, walk or occluded) not yet
     // applied; that happens when the lane takes its next entry (kRefillLanes).
-    bool active = false, exhausted = n == 0, pending = false, overflow = false;
-    while (!__all_sync(full, exhausted)) {
+    bool active = false, pending = false, overflow = false;
+    const int warps = gridDim.x * (256 / 32);
+    bool exhausted = lane >= (n + warps - 1) / warps;
+    bool drained = false;
+    int bound = s0.root.bound, rootRef = s0.root.ref;
+    // Applies the outcome of a lane's traced segment: accepted, to be walked, or occluded.
+    auto settle = [&](bool done) {
+        bool toWalk = false;
+        if (done && !st.found) {
+            if (kWalls && st.crossed) toWalk = true;
+            else shadow_accept<kMedia>(SceneOf<kBatch>::get(s0, scenes, rid), P, S, q);
+        }
+        if (kWalls) {
+            const unsigned m = __ballot_sync(full, toWalk);
+            if (m) {
+                const int leader = __ffs(m) - 1;
+                int wb = 0;
+                if (lane == leader) wb = atomicAdd(counters + kCntWalk, __popc(m));
+                wb = __shfl_sync(full, wb, leader);
+                if (toWalk) S.walk[wb + __popc(m & ((1u << lane) - 1u))] = q;
+            }
+        }
+    };
+    while (true) {
         const bool idle = !active && !exhausted;
         const unsigned need = __ballot_sync(full, idle), busy = __ballot_sync(full, active);
         if (need && (__popc(need) >= kRefillLanes || !busy)) {
-            bool toWalk = false;
-            if (idle && pending && !st.found) {
-                if (kWalls && st.crossed) toWalk = true;
-                else shadow_accept<kMedia>(SceneOf<kBatch>::get(s0, scenes, rid), P, S, q);
-            }
+            settle(idle && pending);
             pending = false;
-            if (kWalls) {
-                const unsigned m = __ballot_sync(full, toWalk);
-                if (m) {
-                    const int leader = __ffs(m) - 1;
-                    int wb = 0;
-                    if (lane == leader) wb = atomicAdd(counters + kCntWalk, __popc(m));
-                    wb = __shfl_sync(full, wb, leader);
-                    if (toWalk) S.walk[wb + __popc(m & ((1u << lane) - 1u))] = q;
-                }
-            }
             int base = 0;
             if (lane == 0) base = atomicAdd(counters + kCntShadowWork, __popc(need));
             base = __shfl_sync(full, base, 0);
@@ -1798,16 +1833,34 @@ __global__ void __launch_bounds__(256, (kSpheres || kMedia || kWalls) ? 1 : 4)
                                        s.root.box[5], &te) &&
                              te < st.tMax;
                     st.ref = s.root.ref;
+                    if (kBatch) {
+                        bound = s.root.bound;
+                        rootRef = s.root.ref;
+                    }
                     // A segment that misses the root box: unoccluded, accepted at the next refill.
                     pending = !active;
                 }
             }
+            drained = __any_sync(full, exhausted) && __all_sync(full, !active || bound <= kCoopBound);
+            continue;
         }
-        if (active && traverse4_step_st<true, kSpheres, kWalls>(nodes, leaves, r, st, hs, &overflow, cls)) {
+        if (!busy) break;
+        if (drained && coop_ready(busy, active, st.sp)) break;
+        bool done = false;
+        if (leaf_turn(busy, __ballot_sync(full, active && st.ref < 0))) {
+            if (active && st.ref < 0) done = traverse4_leaf<true, kSpheres, kWalls, false>(leaves, r, st, hs, cls);
+        } else if (active && st.ref >= 0) {
+            done = traverse4_node<true, false>(nodes, r, st, hs, &overflow);
+        }
+        if (done) {
             active = false;
             pending = true;
         }
     }
+    if (__any_sync(full, active))
+        overflow |= traverse4_finish<true, kSpheres, kWalls, kBatch>(nodes, leaves, cls, bound, rootRef, r, st, active, hs,
+                                                                     1.f - kShadowEps);
+    settle(active || pending);
     if (overflow) atomicOr(counters + kCntStatus, kStatusStack);
 }
 
