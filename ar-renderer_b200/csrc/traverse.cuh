@@ -665,6 +665,9 @@ __device__ __noinline__ CoopState traverse4_coop(const QNode *nodes, const LeafP
     const TraceRay r = make_trace_ray(o, d);
     unsigned rays = __ballot_sync(full, active);
     const int region = __popc(rays & ((1u << lane) - 1u));
+    // The loop's last stores to the columns come before what is written below into other lanes' columns;
+    // the votes alone order no memory, and with empty stacks the loop below has no barrier of its own.
+    __syncwarp();
     // In place: row e is read by every ray before entry e lands in row e / 4.
     for (int e = 0; __any_sync(full, active && e < st.sp); ++e) {
         int2 v = make_int2(0, 0);
