@@ -139,8 +139,9 @@ template <typename K> int resident_blocks(K kernel, int block) {
 constexpr int64_t kTailRays = 3 << 20;
 
 // dStatus points at the accel's 16-byte status block: int status at 0, ray counter at 8.
-// wide: the 4-wide tree (fast; hits identical up to the order among exactly equal distances);
-// otherwise the binary tree in the reference's visit order (bvh.cpp:184-190).
+// wide: the 4-wide tree, each ray's hit a function of the ray and the tree alone; otherwise the binary
+// tree in the reference's visit order (bvh.cpp:184-190). The two visit leaves in different orders, which
+// shows among hits at exactly equal distances, or closer together than the rounding of a box's entry.
 void launch_trace(const DeviceAccel &acc, const prgpu::Ray *dRays, int64_t n, bool anyHit, int32_t *dPrim,
                   float *dT, float *dB1, float *dB2, int *dStatus, cudaStream_t s, int smCount, bool wide) {
     if (n <= 0) return;

@@ -14,11 +14,16 @@
 
 namespace prb {
 
+// RootInfo::bound of a tree with a box that is not within its parent's (or not a number). The cooperative
+// traversal opens nodes ahead of their turn, which keeps the one-lane walk's result only while a child is
+// entered no earlier than its parent: it leaves such trees alone, as it does trees that are too deep.
+constexpr int kLooseBound = 1 << 20;
+
 struct RootInfo {
     float box[6];
     int ref;
     int empty;  // 1 = no nodes: every query misses
-    int bound;  // most entries a depth-first walk of the 4-wide tree holds at a time
+    int bound;  // most entries a depth-first walk of the 4-wide tree holds at a time; kLooseBound: see there
 };
 
 struct HostAccel {
@@ -185,11 +190,17 @@ bool convert_bvh(const prgpu::BVHNode *nodes, int32_t nodeCount, const int32_t *
         const prgpu::BVHNode &n = nodes[c];
         return n.nPrims == 0 ? interiorIndex[size_t(c)] : ~n.offset;
     };
+    auto within = [](const prgpu::BVHNode &c, const prgpu::BVHNode &p) {
+        return c.bmin.x >= p.bmin.x && c.bmin.y >= p.bmin.y && c.bmin.z >= p.bmin.z && c.bmax.x <= p.bmax.x &&
+               c.bmax.y <= p.bmax.y && c.bmax.z <= p.bmax.z;
+    };
+    bool nested = true;
     out->nodes.resize(size_t(nInterior));
     for (int32_t i = 0; i < nodeCount; ++i) {
         const prgpu::BVHNode &n = nodes[i];
         if (n.nPrims != 0) continue;
         const prgpu::BVHNode &a = nodes[i + 1], &b = nodes[n.offset];
+        nested = nested && within(a, n) && within(b, n);
         WNode w;
         w.a = make_float4(a.bmin.x, a.bmin.y, a.bmin.z, a.bmax.x);
         w.b = make_float4(a.bmax.y, a.bmax.z, b.bmin.x, b.bmin.y);
@@ -217,7 +228,8 @@ bool convert_bvh(const prgpu::BVHNode *nodes, int32_t nodeCount, const int32_t *
         out->qnodes.reserve(out->nodes.size() / 2 + 1);
         int levels = 0;
         collapse4(*out, out->root.ref, &out->qnodes, 0, &levels);
-        out->root.bound = 3 * levels + 1;  // a node takes one entry and leaves at most four
+        // A node takes one entry and leaves at most four.
+        out->root.bound = nested ? 3 * levels + 1 : kLooseBound;
     } else {
         out->root.bound = 1;
     }

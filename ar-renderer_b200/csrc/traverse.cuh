@@ -408,8 +408,9 @@ __device__ __forceinline__ bool traverse_step(const WNode *__restrict__ nodes, c
 // The step traversal over the 4-wide tree: the children a node's slab tests accept (entry before
 // tMax) are visited nearest first, the others pushed with their entry distance, farthest first.
 // Box and triangle arithmetic are those of the binary traversal, so a hit's primitive and
-// distance are the reference's; only the order among hits at exactly equal distance can differ
-// (the binary traversal reproduces the reference's visit order for those).
+// distance are the reference's; only among hits at exactly equal distances, or closer together than
+// the rounding of a box's entry, can the visit order tell (the binary traversal reproduces the
+// reference's order for those).
 __device__ __forceinline__ void cswap(float &ta, int &ra, float &tb, int &rb) {
     if (tb < ta) {
         float t = ta;
@@ -419,6 +420,16 @@ __device__ __forceinline__ void cswap(float &ta, int &ra, float &tb, int &rb) {
         ra = rb;
         rb = q;
     }
+}
+
+// Sorting network for 4 (5 compare-exchanges); misses sort last at +inf. Not stable: which of two children
+// entered at the same distance comes first is the network's doing, and part of the visit order.
+__device__ __forceinline__ void sort4(float &t0, int &r0, float &t1, int &r1, float &t2, int &r2, float &t3, int &r3) {
+    cswap(t0, r0, t1, r1);
+    cswap(t2, r2, t3, r3);
+    cswap(t0, r0, t2, r2);
+    cswap(t1, r1, t3, r3);
+    cswap(t1, r1, t2, r2);
 }
 
 // kSkipTransparent: primitives whose class byte (cls) has kTransparentBit do not count as hits;
@@ -543,12 +554,7 @@ __device__ __forceinline__ bool traverse4_node(const QNode *__restrict__ nodes, 
         }
     }
     int r0 = ch.x, r1 = ch.y, r2 = ch.z, r3 = ch.w;
-    // Sorting network for 4 (5 compare-exchanges); misses sort last at +inf.
-    cswap(t0, r0, t1, r1);
-    cswap(t2, r2, t3, r3);
-    cswap(t0, r0, t2, r2);
-    cswap(t1, r1, t3, r3);
-    cswap(t1, r1, t2, r2);
+    sort4(t0, r0, t1, r1, t2, r2, t3, r3);
     if (t0 < inf) {
         const int extra = (t1 < inf) + (t2 < inf) + (t3 < inf);
         if (s.sp + extra > kStackSize) {
@@ -633,10 +639,20 @@ __device__ __forceinline__ Hit finish_hit(const LeafPrim *__restrict__ prims, co
 // back on the stack, so a ray takes a step per level of the tree rather than per node. Measured (B200,
 // closest hit, us, one lane a ray to the end / this): 1,000 rays, 4,096 triangles 81 / 32; 4,096 rays,
 // 100,003 triangles 112 / 56; 1.5M rays, 100,003 triangles 450 / 421.
-// Box and triangle arithmetic are those of the other traversals and a deferred entry is dropped under
-// the same condition, so hits agree up to the order among exactly equal distances. An accepted distance
-// that is not a number (a determinant whose reciprocal overflows) makes the outcome depend on the visit
-// order: such a ray is handed back (true in its lane) for the one-lane traversal to start over.
+//
+// The result is that of the one-lane walk bit for bit, so it does not depend on which rays a warp was left
+// with. Box and triangle arithmetic are those of the other traversals, and for a closest hit the walk's
+// order is kept: an entry above another on a stack comes with all it leads to before it. Nodes may be
+// opened ahead of their turn (an entry is tested against tMax again when it is taken, and tMax only falls;
+// a child lies within its node's box and so is entered no earlier, see kLooseBound; the children are sorted by the one-lane walk's own network, in which entries that fall away later, being
+// farther than all that stay, do not change the order of the rest), but a leaf is tested only once all
+// entries above it are leaves that end in the same step. Of those the hits count in order: a leaf entered
+// at or beyond an earlier leaf's hit is not visited (rounding can put a hit before its own box's entry, so
+// a later hit may be the nearer one and still not count), and equal distances go to the first. What the
+// order of one step cannot settle is handed back (true in its lane) for the one-lane traversal to start
+// over: a nearer hit in such a leaf, an accepted distance that is not a number (a determinant whose
+// reciprocal overflows), and a sphere tied with another hit (its distance is compared in doubles).
+// Any-hit queries take entries in any order: their outcome does not depend on it.
 //
 // The rays' own lanes keep r and st; stacks move in place from the lanes' columns to regions of 64
 // entries (4 columns of the warp's 32, entry e in row e / 4). `bound` is the most entries a depth-first
@@ -723,18 +739,27 @@ __device__ __noinline__ CoopState traverse4_coop(const QNode *nodes, const LeafP
         const int take = min(min(perRay, sp), max(1, (kStackSize - qb - sp) / 3));
         const int turn = group & (perRay - 1);  // 0 takes the topmost entry
         int2 *reg = warpStack + 4 * myRegion;
+        const int quad = lane & ~(kRayLanes - 1);
+        const unsigned lanesOfRay = (perRay == 8 ? full : (1u << (kRayLanes * perRay)) - 1u)
+                                    << (lane & ~(kRayLanes * perRay - 1));
+        const unsigned earlier = lanesOfRay & ((1u << quad) - 1u);  // lanes at entries above this lane's
         int ref = 0;
+        float entry = inf;
         bool work = mine && turn < take;
         if (work) {
             const int e = sp - 1 - turn;
             const int2 v = reg[(e >> 2) * kRow + (e & 3)];
             ref = v.x;
-            work = __int_as_float(v.y) < tMax;
+            entry = __int_as_float(v.y);
+            work = entry < tMax;
         }
+        // Whether a leaf is tested in this step; if not it stays on the stack as it is.
+        bool inTurn = true;
+        if (!kAny && perRay > 1) inTurn = !(__ballot_sync(full, work && ref >= 0) & earlier);
         __syncwarp();
         float t = inf;   // entry distance of the child, or the leaf's own for its next four triangles
         int next = 0;
-        bool hit = false, last = false, nan = false, wall = false;
+        bool hit = false, last = false, nan = false, wall = false, sphere = false, goesOn = false;
         float th = inf;
         if (work) {
             if (ref >= 0) {
@@ -755,16 +780,16 @@ __device__ __noinline__ CoopState traverse4_coop(const QNode *nodes, const LeafP
                     t = box_entry(q, bx ? fx : nx, by ? fy : ny, bz ? fz : nz, bx ? nx : fx, by ? ny : fy, bz ? nz : fz,
                                   &te) && te < tMax ? te : inf;
                 }
-            } else {
+            } else if (inTurn) {
                 // Slots past the leaf's last belong to other leaves or are padding: loaded, not tested.
                 const LeafPrim *p = lp + ~ref + sub;
                 const float4 v0 = __ldg(&p->v0), v1 = __ldg(&p->v1), v2 = __ldg(&p->v2);
                 last = __float_as_int(v2.w) != 0;
-                const unsigned quad = 0xfu << (lane & ~3);
-                const unsigned ends = (__ballot_sync(quad, last) >> (lane & ~3)) & 0xfu;
+                const unsigned ends = (__ballot_sync(0xfu << quad, last) >> quad) & 0xfu;
                 if (ends == 0u || sub < __ffs(ends)) {
                     float u, v;
-                    if (kSpheres && __float_as_int(v1.w) == 1)
+                    sphere = kSpheres && __float_as_int(v1.w) == 1;
+                    if (sphere)
                         hit = hit_sphere(q, v0, v1, tMax, &th);
                     else
                         hit = hit_triangle(q, v0, v1, v2, tMax, &th, &u, &v);
@@ -774,24 +799,49 @@ __device__ __noinline__ CoopState traverse4_coop(const QNode *nodes, const LeafP
                     }
                     nan = hit && !(th == th);
                 }
-                if (ends == 0u && sub == 0) {
+                goesOn = ends == 0u;
+                if (goesOn && sub == 0) {
                     t = -inf;
                     next = ref - kRayLanes;  // ~(slot + 4)
                 }
             }
         }
         __syncwarp();
-        const unsigned lanesOfRay = (perRay == 8 ? full : (1u << (kRayLanes * perRay)) - 1u)
-                                    << (lane & ~(kRayLanes * perRay - 1));
+        if (!kAny && perRay > 1) {
+            // A leaf behind one that goes on was tested too early.
+            if (__ballot_sync(full, goesOn) & earlier) inTurn = false;
+            if (work && ref < 0 && !inTurn) {
+                hit = nan = false;
+                t = sub == 0 ? entry : inf;
+                next = ref;
+            }
+        }
         const int myFirst = __popc(rays & ((1u << lane) - 1u)) * kRayLanes * perRay;  // of the ray this lane owns
         const bool own = (rays >> lane) & 1u;
         const unsigned ownLanes = own ? (perRay == 8 ? full : (1u << (kRayLanes * perRay)) - 1u) << myFirst : 0u;
         const unsigned hits = __ballot_sync(full, hit);
         if (hits) {
             if (!kAny) {
+                // The least distance of each group, of the groups up to it, and of the ray's.
                 float best = hit ? th : inf;
-                for (int k = 1; k < kRayLanes * perRay; k <<= 1) best = fminf(best, __shfl_xor_sync(full, best, k));
+                for (int k = 1; k < kRayLanes; k <<= 1) best = fminf(best, __shfl_xor_sync(full, best, k));
+                bool back = nan;
+                if (perRay > 1) {
+                    for (int k = kRayLanes; k < kRayLanes * perRay; k <<= 1) {
+                        const float o = __shfl_up_sync(full, best, k);
+                        if ((lane & (kRayLanes * perRay - 1)) >= k) best = fminf(best, o);
+                    }
+                    const float above = __shfl_up_sync(full, best, kRayLanes);
+                    const float atTurn = turn > 0 ? fminf(tMax, above) : tMax;  // tMax when the walk comes to this leaf
+                    best = __shfl_sync(full, best, lane | (kRayLanes * perRay - 1));
+                    if (work && ref < 0 && inTurn && !(entry < atTurn)) {  // not visited
+                        back |= hit && th < atTurn;
+                        hit = false;
+                        t = inf;
+                    }
+                }
                 const unsigned win = __ballot_sync(full, hit && th == best);
+                if (kSpheres) back |= sphere && hit && th == best && (win & lanesOfRay & ((1u << lane) - 1u));
                 const unsigned w = win & ownLanes;
                 const int src = w ? __ffs(w) - 1 : 0;
                 const float tb = __shfl_sync(full, th, src);
@@ -799,20 +849,31 @@ __device__ __noinline__ CoopState traverse4_coop(const QNode *nodes, const LeafP
                 if (w) {
                     st.tMax = tb;
                     st.hit.prim = ~rb + (src & (kRayLanes - 1));
+                    st.found = true;
                 }
                 tMax = best < tMax ? best : tMax;
                 if (!(t < tMax)) t = inf;
+                if (__ballot_sync(full, back) & ownLanes) redo = true;
+            } else {
+                if (hits & ownLanes) st.found = true;
             }
-            if (hits & ownLanes) st.found = true;
-            if (__ballot_sync(full, nan) & ownLanes) redo = true;
         }
         if (kSkipTransparent && (__ballot_sync(full, wall) & ownLanes)) st.crossed = true;
         // Push: the later turns' children below the earlier ones', within a group farthest first.
         int rank = 0;
+        bool tie = false;
 #pragma unroll
         for (int k = 1; k < kRayLanes; ++k) {
             const float o = __shfl_xor_sync(full, t, k);
-            rank += o < t || (o == t && (sub ^ k) < sub);
+            rank += o < t || (kAny && o == t && (sub ^ k) < sub);
+            tie |= o == t;
+        }
+        if (!kAny && __any_sync(full, tie && t < inf)) {
+            float t0 = __shfl_sync(full, t, quad), t1 = __shfl_sync(full, t, quad + 1);
+            float t2 = __shfl_sync(full, t, quad + 2), t3 = __shfl_sync(full, t, quad + 3);
+            int i0 = 0, i1 = 1, i2 = 2, i3 = 3;
+            sort4(t0, i0, t1, i1, t2, i2, t3, i3);
+            rank = sub == i1 ? 1 : (sub == i2 ? 2 : (sub == i3 ? 3 : 0));
         }
         const unsigned push = __ballot_sync(full, t < inf);
         if (t < inf) {
