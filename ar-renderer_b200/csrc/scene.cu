@@ -2,12 +2,15 @@
 // checked on the host, so malformed input is an error return, never a device fault), conversion
 // of the BVH, and a content-keyed cache so progressive batches upload once. The reference keys
 // its cache on the primitive pointer and counts only (src/gpu/prender_gpu.cpp:1653-1670) and so
-// misses an edited scene behind the same pointer; here the key also hashes the small tables in
-// full and a strided sample of the large ones.
+// misses an edited scene behind the same pointer; here the key hashes every byte that the device
+// copy is made from.
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
+#include <exception>
+#include <thread>
 #include <vector>
 
 #include "scene.cuh"
@@ -16,10 +19,11 @@ namespace prb {
 
 namespace {
 
+// SceneExt::rgbToSpectrum: 64 z nodes, then coefficients [3][64][64][64][3].
+constexpr size_t kRgbTableFloats = 64 + size_t(3) * 64 * 64 * 64 * 3;
+
 // Content hash, 8 bytes a step in four independent lanes: each step is a bijection of its lane for
-// fixed input and of its input for a fixed lane, so a change of one word always shows. (Byte-wise
-// FNV-1a, the former hash, costs one multiply's latency a byte: over 1 ms for the sampled megabyte of
-// a scene's key, in every render call; this takes a tenth of that.)
+// fixed input and of its input for a fixed lane, so a change of one word always shows.
 struct Hasher {
     uint64_t lane[4] = {0xcbf29ce484222325ull, 0x84222325cbf29ce4ull, 0x9ae16a3b2f90404full, 0xc949d7c7509e6557ull};
     void word(int k, uint64_t w) {
@@ -41,83 +45,146 @@ struct Hasher {
         }
     }
     template <typename T> void value(const T &v) { bytes(&v, sizeof(T)); }
-    // Up to `samples` evenly strided elements plus the last.
-    void sampled(const void *base, size_t count, size_t elem, size_t samples) {
-        value(count);
-        if (!base || count == 0) return;
-        const unsigned char *b = static_cast<const unsigned char *>(base);
-        const size_t step = std::max<size_t>(1, count / samples), ahead = 16 * step;
-        if (elem == sizeof(uint32_t)) {
-            int k = 0;
-            for (size_t i = 0; i < count; i += step, k = (k + 1) & 3) {
-                uint32_t w;
-                std::memcpy(&w, b + i * elem, sizeof(w));
-                word(k, w);
-            }
-        } else {
-            for (size_t i = 0; i < count; i += step) {
-                if (i + ahead < count)
-                    for (size_t c = 0; c < elem; c += 64) __builtin_prefetch(b + (i + ahead) * elem + c);
-                bytes(b + i * elem, elem);
-            }
-        }
-        bytes(b + (count - 1) * elem, elem);
-    }
     uint64_t done() {
         for (int k = 1; k < 4; ++k) word(0, lane[k]);
         return lane[0];
     }
 };
 
-uint64_t scene_key(const prgpu::SceneDesc *sd, const prgpu::SceneExt *ext) {
-    Hasher h;
+// The key's input: small values and arrays in order, and large arrays in blocks that are hashed by
+// several threads and folded in as one word each. The whole content is read in every render call, at
+// memory speed, and only changed content is checked and converted.
+class KeyBuilder {
+  public:
+    template <typename T> void value(const T &v) { small_.value(v); }
+    void array(const void *p, size_t n) {
+        small_.value(n);
+        if (!p) return;
+        const unsigned char *b = static_cast<const unsigned char *>(p);
+        if (n < kBlock / 16) {
+            small_.bytes(b, n);
+            return;
+        }
+        for (size_t i = 0; i < n; i += kBlock) blocks_.push_back({b + i, std::min(kBlock, n - i), 0});
+    }
+    // Starts the hashing on up to `most` other threads; done() takes part in what is left of it. In
+    // between the caller may work on, but not change the arrays.
+    void begin(size_t most) {
+        // A thread takes 17 us to start and join, as long as a block takes to hash: four blocks each. 8 MB
+        // in us over 1 / 4 / 8 / 16 threads: 466 / 156 / 132 / 200; 80 MB: 9073 / 2204 / 1265 / 671.
+        const size_t want = std::min<size_t>(std::min<size_t>(most + 1, std::thread::hardware_concurrency()),
+                                             blocks_.size() / 4);
+        helpers_.reserve(want);
+        try {
+            for (size_t k = 1; k < want; ++k) helpers_.emplace_back([this] { work(); });
+        } catch (const std::exception &) {  // no more threads to be had: those there are do it all
+        }
+    }
+    uint64_t done() {
+        work();
+        join();
+        for (const Block &b : blocks_) small_.value(b.hash);
+        return small_.done();
+    }
+    ~KeyBuilder() {
+        next_ = blocks_.size();  // left early: nothing more is taken
+        join();
+    }
+
+  private:
+    static constexpr size_t kBlock = size_t(1) << 18;
+    struct Block {
+        const unsigned char *p;
+        size_t n;
+        uint64_t hash;
+    };
+    void work() {
+        for (size_t k; (k = next_.fetch_add(1, std::memory_order_relaxed)) < blocks_.size();) {
+            Hasher h;
+            h.bytes(blocks_[k].p, blocks_[k].n);
+            blocks_[k].hash = h.done();
+        }
+    }
+    void join() {
+        for (std::thread &t : helpers_) t.join();
+        helpers_.clear();
+    }
+    Hasher small_;
+    std::vector<Block> blocks_;
+    std::vector<std::thread> helpers_;
+    std::atomic<size_t> next_{0};
+};
+
+bool has_sheen(const prgpu::SceneDesc *sd) {
+    for (int32_t i = 0; i < sd->materialCount; ++i)
+        if (sd->materials[i].sheenWeight > 0 && sd->materials[i].sheenColor >= 0) return true;
+    return false;
+}
+
+// Whether a material names a texture, so that the images and the RGB -> spectrum table are needed.
+bool textures_used(const prgpu::SceneExt *ext) {
+    const int32_t n = ext && ext->textures ? ext->textureCount : 0;
+    const int32_t nm = ext && ext->materialTextures ? ext->materialTextureCount : 0;
+    const int32_t nn = ext && ext->textureNodes ? ext->textureNodeCount : 0;
+    for (int32_t i = 0; i < nm; ++i) {
+        const prgpu::MaterialTextures &x = ext->materialTextures[i];
+        if ((n > 0 && (x.reflectance >= 0 || x.normalMap >= 0 || x.bumpMap >= 0)) ||
+            (nn > 0 && (x.reflectanceNode >= 0 || x.bumpNode >= 0 || x.roughnessNodeU >= 0 || x.roughnessNodeV >= 0 ||
+                        x.coatRoughnessNode >= 0 || x.thicknessNode >= 0 || x.coatAlbedoNode >= 0 ||
+                        x.sheenColorNode >= 0 || x.sheenRoughnessNode >= 0 || x.etaNode >= 0)))
+            return true;
+    }
+    return false;
+}
+
+// Everything that upload_scene's device copy, and the check of the primitives, depend on. The counts
+// and pointers have been checked (validate).
+void scene_key(const prgpu::SceneDesc *sd, const prgpu::SceneExt *ext, KeyBuilder &h) {
     h.value(sd->prims);
     h.value(sd->nodes);
-    h.value(sd->primCount);
-    h.value(sd->nodeCount);
-    h.sampled(sd->prims, size_t(sd->primCount), sizeof(prgpu::Primitive), 4096);
-    h.sampled(sd->nodes, size_t(sd->nodeCount), sizeof(prgpu::BVHNode), 4096);
-    h.sampled(sd->primOrder, size_t(sd->primCount), sizeof(int32_t), 4096);
-    if (sd->materials) h.bytes(sd->materials, size_t(sd->materialCount) * sizeof(prgpu::Material));
-    if (sd->lights) h.bytes(sd->lights, size_t(sd->lightCount) * sizeof(prgpu::Light));
-    if (sd->spectra) h.bytes(sd->spectra, size_t(sd->spectrumCount) * sizeof(prgpu::Spectrum));
-    if (sd->media) h.bytes(sd->media, size_t(sd->mediumCount) * sizeof(prgpu::Medium));
-    h.bytes(sd->filter.cdf, sizeof(sd->filter.cdf));
+    h.array(sd->prims, size_t(sd->primCount) * sizeof(prgpu::Primitive));
+    h.array(sd->nodes, size_t(sd->nodeCount) * sizeof(prgpu::BVHNode));
+    h.array(sd->primOrder, size_t(sd->primCount) * sizeof(int32_t));
+    h.array(sd->materials, size_t(sd->materialCount) * sizeof(prgpu::Material));
+    h.array(sd->lights, size_t(sd->lightCount) * sizeof(prgpu::Light));
+    h.array(sd->spectra, size_t(sd->spectrumCount) * sizeof(prgpu::Spectrum));
+    h.array(sd->media, size_t(sd->mediumCount) * sizeof(prgpu::Medium));
+    h.array(sd->filter.cdf, sizeof(sd->filter.cdf));
+    if (has_sheen(sd)) h.array(sd->sheenAlbedo, size_t(prgpu::kSheenAlpha) * prgpu::kSheenMu * sizeof(float));
     if (ext && ext->lightBVH && ext->lightBVHNodeCount > 0)
-        h.bytes(ext->lightBVH, size_t(ext->lightBVHNodeCount) * sizeof(prgpu::LightBVHNode));
+        h.array(ext->lightBVH, size_t(ext->lightBVHNodeCount) * sizeof(prgpu::LightBVHNode));
     if (ext && ext->envMap) {
         h.value(*ext->envMap);
-        h.sampled(ext->envMap->texels, size_t(std::max(0, ext->envMap->width)) * size_t(std::max(0, ext->envMap->height)),
-                        4 * sizeof(float), 65536);
+        h.array(ext->envMap->texels, size_t(ext->envMap->width) * size_t(ext->envMap->height) * 4 * sizeof(float));
+        h.array(sd->cie, size_t(3) * prgpu::kSpectrumSamples * sizeof(float));
     }
     if (ext && ext->sun) h.value(*ext->sun);
     if (ext && ext->textureNodes && ext->textureNodeCount > 0)
-        h.bytes(ext->textureNodes, size_t(ext->textureNodeCount) * sizeof(prgpu::TextureNode));
+        h.array(ext->textureNodes, size_t(ext->textureNodeCount) * sizeof(prgpu::TextureNode));
     if (ext && ((ext->textures && ext->textureCount > 0) || (ext->textureNodes && ext->textureNodeCount > 0))) {
         for (int32_t k = 0; ext->textures && k < ext->textureCount; ++k) {
             const prgpu::ImageTextureDesc &t = ext->textures[k];
             h.value(t);
-            h.sampled(t.rgb, size_t(std::max(0, t.width)) * size_t(std::max(0, t.height)), 3 * sizeof(float), 65536);
+            h.array(t.rgb, size_t(t.width) * size_t(t.height) * 3 * sizeof(float));
         }
         if (ext->materialTextures && ext->materialTextureCount > 0)
-            h.bytes(ext->materialTextures, size_t(ext->materialTextureCount) * sizeof(prgpu::MaterialTextures));
-        h.value(ext->rgbToSpectrum);
+            h.array(ext->materialTextures, size_t(ext->materialTextureCount) * sizeof(prgpu::MaterialTextures));
+        if (textures_used(ext)) h.array(ext->rgbToSpectrum, kRgbTableFloats * sizeof(float));
     }
     if (ext && ext->deltaLights && ext->deltaLightCount > 0)
         for (int32_t k = 0; k < ext->deltaLightCount; ++k) {
             const prgpu::DeltaLightDesc &l = ext->deltaLights[k];
             h.value(l);
-            if (l.type == prgpu::DeltaGoniometric && l.profile && l.nV > 0 && l.nH > 0)
-                h.bytes(l.profile, (size_t(l.nV) + size_t(l.nH) + size_t(l.nV) * size_t(l.nH)) * sizeof(float));
+            if (l.type == prgpu::DeltaGoniometric)
+                h.array(l.profile, (size_t(l.nV) + size_t(l.nH) + size_t(l.nV) * size_t(l.nH)) * sizeof(float));
         }
+    h.value(ext ? ext->gridMediumCount : 0);
     if (ext && ext->gridMedia && ext->gridMediumCount > 0)
         for (int32_t k = 0; k < ext->gridMediumCount; ++k) {
             const prgpu::GridMediumDesc &g = ext->gridMedia[k];
             h.value(g);
-            if (g.field != prgpu::GridNoise)
-                h.sampled(g.density, size_t(g.nx) * size_t(g.ny) * size_t(g.nz), sizeof(float), 65536);
+            if (g.field != prgpu::GridNoise) h.array(g.density, size_t(g.nx) * size_t(g.ny) * size_t(g.nz) * sizeof(float));
         }
-    return h.done();
 }
 
 bool spec_ok(int32_t id, int32_t n) { return id >= -1 && id < n; }
@@ -159,6 +226,7 @@ bool texture_tree_has_image(const prgpu::SceneExt *ext, int32_t node, int depth)
     return false;
 }
 
+// All of a scene but its primitives.
 bool validate(const prgpu::SceneDesc *sd, const prgpu::SceneExt *ext, std::string *err) {
     auto fail = [&](const std::string &m) {
         *err = m;
@@ -298,14 +366,6 @@ bool validate(const prgpu::SceneDesc *sd, const prgpu::SceneExt *ext, std::strin
     for (int32_t i = 0; i < sd->mediumCount; ++i)
         if (!spec_ok(sd->media[i].sigmaA, ns) || !spec_ok(sd->media[i].sigmaS, ns))
             return fail("medium spectrum index out of range");
-    for (int32_t i = 0; i < sd->primCount; ++i) {
-        const prgpu::Primitive &p = sd->prims[i];
-        if (p.type > prgpu::PrimSphere) return fail("unknown primitive type");
-        if (p.material < 0 || p.material >= sd->materialCount) return fail("primitive material out of range");
-        if (p.light < -1 || p.light >= sd->lightCount) return fail("primitive light out of range");
-        if (p.mediumInside < -1 || p.mediumInside >= nm || p.mediumOutside < -1 || p.mediumOutside >= nm)
-            return fail("primitive medium out of range");
-    }
     if (ext && ext->lightBVHNodeCount > 0) {
         if (!ext->lightBVH) return fail("null light BVH");
         int32_t n = ext->lightBVHNodeCount;
@@ -317,6 +377,25 @@ bool validate(const prgpu::SceneDesc *sd, const prgpu::SceneExt *ext, std::strin
                 return fail("malformed light BVH interior node");
             }
             if (b.parent >= i || b.parent < -1 || (i > 0 && b.parent < 0)) return fail("malformed light BVH parent link");
+        }
+    }
+    return true;
+}
+
+// The primitives' part of the check, for content that the device does not hold yet.
+bool validate_prims(const prgpu::SceneDesc *sd, const prgpu::SceneExt *ext, std::string *err) {
+    const int32_t nm = sd->mediumCount + (ext && ext->gridMediumCount > 0 ? ext->gridMediumCount : 0);
+    for (int32_t i = 0; i < sd->primCount; ++i) {
+        const prgpu::Primitive &p = sd->prims[i];
+        const char *what = nullptr;
+        if (p.type > prgpu::PrimSphere) what = "unknown primitive type";
+        else if (p.material < 0 || p.material >= sd->materialCount) what = "primitive material out of range";
+        else if (p.light < -1 || p.light >= sd->lightCount) what = "primitive light out of range";
+        else if (p.mediumInside < -1 || p.mediumInside >= nm || p.mediumOutside < -1 || p.mediumOutside >= nm)
+            what = "primitive medium out of range";
+        if (what) {
+            *err = what;
+            return false;
         }
     }
     return true;
@@ -437,15 +516,7 @@ void upload_textures(const prgpu::SceneExt *ext, SceneCache &cache, DevScene &d,
     const int32_t n = ext && ext->textures ? ext->textureCount : 0;
     const int32_t nm = ext && ext->materialTextures ? ext->materialTextureCount : 0;
     const int32_t nn = ext && ext->textureNodes ? ext->textureNodeCount : 0;
-    bool used = false;
-    for (int32_t i = 0; i < nm; ++i) {
-        const prgpu::MaterialTextures &x = ext->materialTextures[i];
-        used = used || (n > 0 && (x.reflectance >= 0 || x.normalMap >= 0 || x.bumpMap >= 0)) ||
-               (nn > 0 && (x.reflectanceNode >= 0 || x.bumpNode >= 0 || x.roughnessNodeU >= 0 || x.roughnessNodeV >= 0 ||
-                           x.coatRoughnessNode >= 0 || x.thicknessNode >= 0 || x.coatAlbedoNode >= 0 ||
-                           x.sheenColorNode >= 0 || x.sheenRoughnessNode >= 0 || x.etaNode >= 0));
-    }
-    if (!used) return;
+    if (!textures_used(ext)) return;
     size_t total = 0;
     for (int32_t k = 0; k < n; ++k) total += size_t(ext->textures[k].width) * ext->textures[k].height * 3;
     cache.texData.ensure(total * sizeof(float));
@@ -485,8 +556,7 @@ void upload_textures(const prgpu::SceneExt *ext, SceneCache &cache, DevScene &d,
     put(cache.matTex, mt.data(), mt.size(), s);
     if (nn > 0) put(cache.texNodes, ext->textureNodes, size_t(nn), s);
     if (ext->rgbToSpectrum) {
-        const size_t tableFloats = 64 + size_t(3) * 64 * 64 * 64 * 3;
-        put(cache.rgbTable, ext->rgbToSpectrum, tableFloats, s);
+        put(cache.rgbTable, ext->rgbToSpectrum, kRgbTableFloats, s);
     }
     PRB_CUDA(cudaStreamSynchronize(s));
     d.textures = n > 0 ? cache.textures.as<DevTex>() : nullptr;
@@ -628,9 +698,19 @@ void upload_env(const prgpu::SceneExt *ext, const prgpu::SceneDesc *sd, SceneCac
 bool upload_scene(DeviceState &ds, const prgpu::SceneDesc *sd, const prgpu::SceneExt *ext, SceneCache &cache,
                   std::string *err) {
     if (!validate(sd, ext, err)) return false;
-    uint64_t key = scene_key(sd, ext);
+    KeyBuilder builder;
+    scene_key(sd, ext, builder);
+    // Another scene by its arrays' places or sizes is hashed while it is converted and uploaded, for which
+    // two threads are enough; else the key decides, and all there are hash.
+    const bool early = cache.valid && cache.hostPrims == sd->prims && cache.hostNodes == sd->nodes &&
+                       cache.primCount == sd->primCount && cache.nodeCount == sd->nodeCount;
+    builder.begin(early ? 15 : 2);
+    const uint64_t key = early ? builder.done() : 0;
+    const bool held = early && cache.key == key;
     DevScene &d = cache.ds;
-    if (!cache.valid || cache.key != key) {
+    if (!held) {
+        // An equal key is equal content, whose primitives were checked when it was uploaded.
+        if (!validate_prims(sd, ext, err)) return false;
         HostAccel h;
         if (!convert_bvh(sd->nodes, sd->nodeCount, sd->primOrder, sd->primCount, PrimitiveSource{sd->prims}, &h, err))
             return false;
@@ -657,9 +737,7 @@ bool upload_scene(DeviceState &ds, const prgpu::SceneDesc *sd, const prgpu::Scen
         }
         cache.wallCount = walls.size() <= size_t(kMaxWallList) ? int(walls.size()) : -1;
         if (cache.wallCount > 0) put(cache.walls, walls.data(), walls.size(), s);
-        cache.hasSheen = false;
-        for (int32_t i = 0; i < sd->materialCount; ++i)
-            if (sd->materials[i].sheenWeight > 0 && sd->materials[i].sheenColor >= 0) cache.hasSheen = true;
+        cache.hasSheen = has_sheen(sd);
         if (cache.hasSheen) {
             std::vector<float> table = sd->sheenAlbedo
                                            ? std::vector<float>(sd->sheenAlbedo, sd->sheenAlbedo + prgpu::kSheenAlpha * prgpu::kSheenMu)
@@ -782,7 +860,11 @@ bool upload_scene(DeviceState &ds, const prgpu::SceneDesc *sd, const prgpu::Scen
         cache.hasSpheres = false;
         for (int32_t i = 0; i < sd->primCount; ++i)
             if (sd->prims[i].type == prgpu::PrimSphere) cache.hasSpheres = true;
-        cache.key = key;
+        cache.key = early ? key : builder.done();
+        cache.hostPrims = sd->prims;
+        cache.hostNodes = sd->nodes;
+        cache.primCount = sd->primCount;
+        cache.nodeCount = sd->nodeCount;
         cache.valid = true;
         cache.deviceBytes = cache.accel.bytes + int64_t(sd->primCount) * int64_t(sizeof(prgpu::Primitive));
         d.nodes = cache.accel.nodes.as<WNode>();

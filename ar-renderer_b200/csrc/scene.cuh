@@ -155,7 +155,9 @@ struct DevScene {
 };
 
 struct SceneCache {
-    uint64_t key = 0;
+    uint64_t key = 0;  // of the content; two scenes at other places or of other sizes differ without it
+    const void *hostPrims = nullptr, *hostNodes = nullptr;
+    int32_t primCount = 0, nodeCount = 0;
     bool valid = false;
     DeviceAccel accel;
     DevBuf prims, primClass, mats, lights, spectra, media, filterCdf, lbvh, lightLeaf, grids, gridData, envTexels,
