@@ -715,6 +715,7 @@ bool upload_scene(DeviceState &ds, const prgpu::SceneDesc *sd, const prgpu::Scen
         if (!convert_bvh(sd->nodes, sd->nodeCount, sd->primOrder, sd->primCount, PrimitiveSource{sd->prims}, &h, err))
             return false;
         cudaStream_t s = ds.stream;
+        cache.valid = false;  // until all of it is there: an upload that throws leaves nothing to reuse
         cache.accel.upload(h, s);
         put(cache.prims, sd->prims, size_t(sd->primCount), s);
         std::vector<uint8_t> cls(size_t(std::max(1, sd->primCount)), uint8_t(kClassOther));
