@@ -502,6 +502,9 @@ PRGPU_API int prgpu_render_aov(int deviceIndex, const prgpu::SceneDesc *sd, cons
     } catch (const CudaError &ce) {
         set_err(err, errLen, ce.msg);
         return 1;
+    } catch (const std::exception &ex) {
+        set_err(err, errLen, ex.what());
+        return 1;
     }
 }
 
