@@ -4,6 +4,7 @@
 // results written as coalesced 4-byte stores.
 
 #include <algorithm>
+#include <map>
 #include <memory>
 
 #include "accel.cuh"
@@ -125,11 +126,41 @@ __global__ void __launch_bounds__(256, 4) k_trace_persist(const void *__restrict
     if (overflow) atomicOr(status, 1);
 }
 
-// Resident blocks per SM of a kernel (cached): the persistent grid is exactly one full wave.
-template <typename K> int resident_blocks(K kernel, int block) {
-    int n = 0;
-    PRB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, block, 0));
-    return std::max(1, n);
+// Resident blocks per SM of a kernel (asked once): the persistent grid is exactly one full wave.
+template <bool kAny, bool kWide, bool kTail> int resident_blocks(int block) {
+    static const int n = [block] {
+        int k = 0;
+        PRB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, k_trace_persist<kAny, kWide, kTail>, block, 0));
+        return std::max(1, k);
+    }();
+    return n;
+}
+
+// A query: device pointers, its status word, and a ray counter that no query that may run at the same
+// time uses (RayCounters).
+struct TraceArgs {
+    const prgpu::Ray *rays;
+    int64_t n;
+    int32_t *prim;
+    float *t, *b1, *b2;
+    int *status;
+    unsigned long long *counter;
+    cudaStream_t stream;
+    int smCount;
+};
+
+// raysPerBlock: one ray a lane, or (tail form) down to one a warp.
+template <bool kAny, bool kWide, bool kTail> void launch_one(const DeviceAccel &acc, const TraceArgs &q) {
+    const int block = 256, raysPerBlock = kTail ? block / 32 : block;
+    const int64_t needed = (q.n + raysPerBlock - 1) / raysPerBlock;
+    const int grid = int(std::min<int64_t>(needed, int64_t(q.smCount) * resident_blocks<kAny, kWide, kTail>(block)));
+    PRB_CUDA(cudaMemsetAsync(q.counter, 0, sizeof(*q.counter), q.stream));
+    k_trace_persist<kAny, kWide, kTail><<<grid, block, 0, q.stream>>>(
+        kWide ? acc.qnodes.ptr : acc.nodes.ptr, acc.prims.as<LeafPrim>(), acc.root,
+        reinterpret_cast<const float4 *>(q.rays), q.n, q.prim, kAny ? nullptr : q.t, kAny ? nullptr : q.b1,
+        kAny ? nullptr : q.b2, q.status, q.counter);
+    count_launch();
+    PRB_CUDA(cudaGetLastError());
 }
 
 // Up to this many rays the launch's tail, 40 to 80 us with one lane a ray to the end, costs more than
@@ -138,40 +169,76 @@ template <typename K> int resident_blocks(K kernel, int block) {
 // 16.8M 4187 / 3897.
 constexpr int64_t kTailRays = 3 << 20;
 
-// dStatus points at the accel's 16-byte status block: int status at 0, ray counter at 8.
 // wide: the 4-wide tree, each ray's hit a function of the ray and the tree alone; otherwise the binary
 // tree in the reference's visit order (bvh.cpp:184-190). The two visit leaves in different orders, which
 // shows among hits at exactly equal distances, or closer together than the rounding of a box's entry.
-void launch_trace(const DeviceAccel &acc, const prgpu::Ray *dRays, int64_t n, bool anyHit, int32_t *dPrim,
-                  float *dT, float *dB1, float *dB2, int *dStatus, cudaStream_t s, int smCount, bool wide) {
-    if (n <= 0) return;
-    const int block = 256;
-    const auto *r4 = reinterpret_cast<const float4 *>(dRays);
-    auto *counter = reinterpret_cast<unsigned long long *>(reinterpret_cast<char *>(dStatus) + 8);
-    PRB_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), s));
-    // Blocks needed at one lane a ray, or (tail form) down to one ray a warp.
-    auto launch = [&](auto kernel, int &resident, const void *nodes, int raysPerBlock) {
-        if (!resident) resident = resident_blocks(kernel, block);
-        const int64_t needed = (n + raysPerBlock - 1) / raysPerBlock;
-        const int grid = int(std::min<int64_t>(needed, int64_t(smCount) * resident));
-        kernel<<<grid, block, 0, s>>>(nodes, acc.prims.as<LeafPrim>(), acc.root, r4, n, dPrim, anyHit ? nullptr : dT,
-                                      anyHit ? nullptr : dB1, anyHit ? nullptr : dB2, dStatus, counter);
-    };
-    static int resident[2][3] = {};
-    const void *q = acc.qnodes.ptr, *w = acc.nodes.ptr;
+void launch_trace(const DeviceAccel &acc, const TraceArgs &q, bool anyHit, bool wide) {
+    if (q.n <= 0) return;
     if (!wide) {
-        if (anyHit) launch(k_trace_persist<true, false, false>, resident[1][0], w, block);
-        else launch(k_trace_persist<false, false, false>, resident[0][0], w, block);
-    } else if (n <= kTailRays) {
-        if (anyHit) launch(k_trace_persist<true, true, true>, resident[1][1], q, block / 32);
-        else launch(k_trace_persist<false, true, true>, resident[0][1], q, block / 32);
+        if (anyHit) launch_one<true, false, false>(acc, q);
+        else launch_one<false, false, false>(acc, q);
+    } else if (q.n <= kTailRays) {
+        if (anyHit) launch_one<true, true, true>(acc, q);
+        else launch_one<false, true, true>(acc, q);
     } else {
-        if (anyHit) launch(k_trace_persist<true, true, false>, resident[1][2], q, block);
-        else launch(k_trace_persist<false, true, false>, resident[0][2], q, block);
+        if (anyHit) launch_one<true, true, false>(acc, q);
+        else launch_one<false, true, false>(acc, q);
     }
-    count_launch();
-    PRB_CUDA(cudaGetLastError());
 }
+
+// The ray counters of a handle. A query resets its counter and draws its rays from it, so queries that
+// may overlap on the device need one each, while those of one stream run one after another and share
+// one: a counter per stream, by the stream's id, which is never used again (its address is). What is
+// captured runs later, on any stream and any number of times: a counter of its own for each such query.
+class RayCounters {
+  public:
+    // The first `count` counters lie in the caller's memory at p, kStride bytes each.
+    static constexpr size_t kStride = 32;
+    void init(void *p, size_t count) {
+        next_ = static_cast<char *>(p);
+        left_ = count;
+    }
+    unsigned long long *of(cudaStream_t stream) {
+        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+        PRB_CUDA(cudaStreamIsCapturing(stream, &capturing));
+        if (capturing != cudaStreamCaptureStatusNone) return take();
+        unsigned long long id = 0;
+        PRB_CUDA(cudaStreamGetId(stream, &id));
+        unsigned long long *&c = known_[id];
+        if (!c) c = take();
+        return c;
+    }
+    void release() {
+        for (DevBuf &b : more_) b.release();
+        more_.clear();
+        known_.clear();
+    }
+
+  private:
+    unsigned long long *take() {
+        if (!left_) grow();
+        auto *c = reinterpret_cast<unsigned long long *>(next_);
+        next_ += kStride;
+        --left_;
+        return c;
+    }
+    void grow() {
+        const size_t count = 4096;
+        more_.emplace_back();
+        // Also while this or another thread captures: an allocation is no part of what is captured.
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        PRB_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+        const cudaError_t e = cudaMalloc(&more_.back().ptr, count * kStride);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) more_.pop_back();
+        check_cuda(e, "cudaMalloc of ray counters");
+        init(more_.back().ptr, count);
+    }
+    std::map<unsigned long long, unsigned long long *> known_;
+    std::vector<DevBuf> more_;
+    char *next_ = nullptr;
+    size_t left_ = 0;
+};
 
 } // namespace prb
 
@@ -180,8 +247,22 @@ using namespace prb;
 struct prgpu_accel_t {
     DeviceAccel acc;
     int device = -1;
-    DevBuf status;
+    DevBuf status;  // two status words (queries on device buffers, on host buffers), then ray counters
     DevBuf rays, prim, t, b1, b2;  // staging for the host-buffer path
+    std::mutex mutex;              // the counters, and a counter's reset with the launch that draws from it
+    RayCounters counters;
+    std::atomic<int> hostStatus{0};  // what host-buffer queries reported, for prgpu_accel_status
+
+    void trace(TraceArgs q, bool anyHit, bool wide) {
+        std::lock_guard<std::mutex> lock(mutex);
+        q.counter = counters.of(q.stream);
+        launch_trace(acc, q, anyHit, wide);
+    }
+    void release() {
+        acc.release();
+        counters.release();
+        for (DevBuf *b : {&status, &rays, &prim, &t, &b1, &b2}) b->release();
+    }
 };
 
 namespace {
@@ -197,8 +278,10 @@ bool make_accel(int deviceIndex, const prgpu::BVHNode *nodes, int32_t nodeCount,
     DeviceState &ds = device_state(deviceIndex);
     a->device = ds.device;
     a->acc.upload(h, ds.stream);
-    a->status.ensure(16);  // status word at 0, persistent-kernel ray counter at 8
-    PRB_CUDA(cudaMemsetAsync(a->status.ptr, 0, 16, ds.stream));
+    const size_t counters = 255;
+    a->status.ensure((1 + counters) * RayCounters::kStride);
+    a->counters.init(a->status.as<char>() + RayCounters::kStride, counters);
+    PRB_CUDA(cudaMemsetAsync(a->status.ptr, 0, 2 * sizeof(int), ds.stream));
     PRB_CUDA(cudaStreamSynchronize(ds.stream));
     return true;
 }
@@ -218,7 +301,8 @@ bool trace_host(prgpu_accel_t *a, const prgpu::Ray *rays, int64_t n, int anyHit,
     if (tOut) a->t.ensure(size_t(std::max<int64_t>(cap, 1)) * sizeof(float));
     if (b1Out) a->b1.ensure(size_t(std::max<int64_t>(cap, 1)) * sizeof(float));
     if (b2Out) a->b2.ensure(size_t(std::max<int64_t>(cap, 1)) * sizeof(float));
-    PRB_CUDA(cudaMemsetAsync(a->status.ptr, 0, sizeof(int), ds.stream));
+    int *dStatus = a->status.as<int>() + 1;
+    PRB_CUDA(cudaMemsetAsync(dStatus, 0, sizeof(int), ds.stream));
     cudaEvent_t copied[2], traced[2];
     for (int k = 0; k < 2; ++k) {
         PRB_CUDA(cudaEventCreateWithFlags(&copied[k], cudaEventDisableTiming));
@@ -235,10 +319,10 @@ bool trace_host(prgpu_accel_t *a, const prgpu::Ray *rays, int64_t n, int anyHit,
                                  cudaMemcpyHostToDevice, ds.copy));
         PRB_CUDA(cudaEventRecord(copied[slot], ds.copy));
         PRB_CUDA(cudaStreamWaitEvent(ds.stream, copied[slot], 0));
-        launch_trace(a->acc, a->rays.as<prgpu::Ray>() + base, cnt, anyHit != 0, a->prim.as<int32_t>() + base,
-                     tOut ? a->t.as<float>() + base : nullptr, b1Out ? a->b1.as<float>() + base : nullptr,
-                     b2Out ? a->b2.as<float>() + base : nullptr, a->status.as<int>(), ds.stream,
-                     ds.prop.multiProcessorCount, wide);
+        a->trace({a->rays.as<prgpu::Ray>() + base, cnt, a->prim.as<int32_t>() + base,
+                  tOut ? a->t.as<float>() + base : nullptr, b1Out ? a->b1.as<float>() + base : nullptr,
+                  b2Out ? a->b2.as<float>() + base : nullptr, dStatus, nullptr, ds.stream, ds.prop.multiProcessorCount},
+                 anyHit != 0, wide);
         PRB_CUDA(cudaMemcpyAsync(primOut + off, a->prim.as<int32_t>() + base, size_t(cnt) * sizeof(int32_t),
                                  cudaMemcpyDeviceToHost, ds.stream));
         if (tOut)
@@ -253,13 +337,14 @@ bool trace_host(prgpu_accel_t *a, const prgpu::Ray *rays, int64_t n, int anyHit,
         PRB_CUDA(cudaEventRecord(traced[slot], ds.stream));
     }
     int status = 0;
-    PRB_CUDA(cudaMemcpyAsync(&status, a->status.ptr, sizeof(int), cudaMemcpyDeviceToHost, ds.stream));
+    PRB_CUDA(cudaMemcpyAsync(&status, dStatus, sizeof(int), cudaMemcpyDeviceToHost, ds.stream));
     PRB_CUDA(cudaStreamSynchronize(ds.stream));
     PRB_CUDA(cudaStreamSynchronize(ds.copy));
     for (int k = 0; k < 2; ++k) {
         cudaEventDestroy(copied[k]);
         cudaEventDestroy(traced[k]);
     }
+    a->hostStatus |= status;
     if (status & 1) {
         *err = "BVH deeper than the traversal stack (64 entries)";
         return false;
@@ -283,13 +368,7 @@ PRGPU_API int prgpu_trace_rays(int deviceIndex, const prgpu::BVHNode *nodes, int
         std::string e;
         bool ok = make_accel(deviceIndex, nodes, nodeCount, primOrder, triVerts, primCount, &a, &e) &&
                   trace_host(&a, rays, rayCount, anyHit, primOut, tOut, b1Out, b2Out, false, &e);
-        a.acc.release();
-        a.status.release();
-        a.rays.release();
-        a.prim.release();
-        a.t.release();
-        a.b1.release();
-        a.b2.release();
+        a.release();
         if (!ok) {
             set_err(err, errLen, e);
             return 1;
@@ -339,11 +418,15 @@ PRGPU_API int prgpu_accel_trace(prgpu_accel accel, const prgpu::Ray *deviceRays,
     }
     try {
         DeviceState &ds = device_state(accel->device);
-        launch_trace(accel->acc, deviceRays, rayCount, anyHit != 0, devicePrimOut, deviceTOut, nullptr, nullptr,
-                     accel->status.as<int>(), static_cast<cudaStream_t>(stream), ds.prop.multiProcessorCount, true);
+        accel->trace({deviceRays, rayCount, devicePrimOut, deviceTOut, nullptr, nullptr, accel->status.as<int>(), nullptr,
+                      static_cast<cudaStream_t>(stream), ds.prop.multiProcessorCount},
+                     anyHit != 0, true);
         return 0;
     } catch (const CudaError &e) {
         set_err(err, errLen, e.msg);
+        return 1;
+    } catch (const std::exception &e) {
+        set_err(err, errLen, e.what());
         return 1;
     }
 }
@@ -367,19 +450,23 @@ PRGPU_API int prgpu_accel_trace_host(prgpu_accel accel, const prgpu::Ray *rays, 
     } catch (const CudaError &e) {
         set_err(err, errLen, e.msg);
         return 1;
+    } catch (const std::exception &e) {
+        set_err(err, errLen, e.what());
+        return 1;
     }
 }
 
-// Reads back and clears the accel's status word (bit 0: a traversal stack overflowed).
+// Reads back and clears the accel's status (bit 0: a traversal stack overflowed), once all queries queued
+// so far, on whatever stream, have run.
 PRGPU_API int prgpu_accel_status(prgpu_accel accel) {
     if (!accel) return -1;
     try {
-        DeviceState &ds = device_state(accel->device);
+        device_state(accel->device);
         int s = 0;
-        PRB_CUDA(cudaStreamSynchronize(ds.stream));
+        PRB_CUDA(cudaDeviceSynchronize());
         PRB_CUDA(cudaMemcpy(&s, accel->status.ptr, sizeof(int), cudaMemcpyDeviceToHost));
-        PRB_CUDA(cudaMemset(accel->status.ptr, 0, sizeof(int)));
-        return s;
+        if (s) PRB_CUDA(cudaMemset(accel->status.ptr, 0, sizeof(int)));
+        return s | accel->hostStatus.exchange(0);
     } catch (const CudaError &) {
         return -1;
     }
@@ -391,12 +478,6 @@ PRGPU_API void prgpu_accel_destroy(prgpu_accel accel) {
     if (!accel) return;
     std::lock_guard<std::mutex> lock(gApiMutex);
     if (accel->device >= 0) cudaSetDevice(accel->device);
-    accel->acc.release();
-    accel->status.release();
-    accel->rays.release();
-    accel->prim.release();
-    accel->t.release();
-    accel->b1.release();
-    accel->b2.release();
+    accel->release();
     delete accel;
 }

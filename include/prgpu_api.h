@@ -536,7 +536,9 @@ PRGPU_API int prgpu_trace_rays_noalloc(int deviceIndex, const prgpu::BVHNode *no
                                        float *tOut, float *b1Out, float *b2Out, char *err, int errLen);
 
 // Device-resident acceleration structure for repeated queries: built once from the same inputs
-// as prgpu_trace_rays, queried with device pointers on a caller stream (cudaStream_t as void*).
+// as prgpu_trace_rays, queried with device pointers on a caller stream (cudaStream_t as void*). One
+// handle takes queries from any number of threads and streams at a time, captured ones included. A hit
+// is a function of the ray and the tree alone, the same in every query that holds the ray.
 typedef struct prgpu_accel_t *prgpu_accel;
 PRGPU_API int prgpu_accel_create(int deviceIndex, const prgpu::BVHNode *nodes, int32_t nodeCount,
                                  const int32_t *primOrder, const prgpu::Float3 *triVerts, int32_t primCount,
@@ -548,7 +550,7 @@ PRGPU_API int prgpu_accel_trace(prgpu_accel accel, const prgpu::Ray *deviceRays,
 PRGPU_API int prgpu_accel_trace_host(prgpu_accel accel, const prgpu::Ray *rays, int64_t rayCount, int32_t anyHit,
                                      int32_t *primOut, float *tOut, char *err, int errLen);
 // Returns and clears the handle's status word: bit 0 = a traversal stack overflowed (the BVH is
-// deeper than 64 levels along some ray); -1 on a bad handle.
+// deeper than 64 levels along some ray); -1 on a bad handle. Waits for the device.
 PRGPU_API int prgpu_accel_status(prgpu_accel accel);
 // Bytes of the converted node and triangle arrays on the device (for roofline accounting).
 PRGPU_API int64_t prgpu_accel_bytes(prgpu_accel accel);
