@@ -1190,8 +1190,10 @@ __global__ void __launch_bounds__(256) k_classify(DevScene s0, const DevScene *s
 // different numbers of steps. A finished lane's hit is stored when it takes its next entry.
 template <bool kSpheres, bool kBatch = false>
 // 4 resident blocks (64 registers) for triangle scenes; the batched form would otherwise take 74
-// registers and 3 blocks. Scenes with spheres keep the double-precision sphere test unconstrained.
-__global__ void __launch_bounds__(256, kSpheres ? 1 : 4) k_extend(DevScene s0, const DevScene *scenes, Paths P,
+// registers and 3 blocks. Scenes with spheres need room for the double-precision sphere test: 3 blocks
+// (80 registers), batched 2. Without a bound the call of traverse4_finish decides: 118, 2 blocks. Box with
+// 60 analytic spheres, 384^2 x 16 samples, with k_shadow_any's bound below: 12.8 -> 11.8 ms.
+__global__ void __launch_bounds__(256, kSpheres ? (kBatch ? 2 : 3) : 4) k_extend(DevScene s0, const DevScene *scenes, Paths P,
                                                                   int *counters, const int *queue) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -1757,8 +1759,12 @@ __device__ __forceinline__ void shadow_accept(const DevScene &s, const Paths &P,
 // registers for the ratio-tracking code). kWalls: the scene has medium interfaces; they are
 // transparent to this query, an occluded segment is done, an unoccluded one that crossed no
 // interface stays in its starting medium, and the rest go to the walk queue (k_shadow_walk).
+// Resident blocks: 4 for triangles alone, 3 with spheres (80 registers), 2 with media or interfaces (128),
+// whose transmittance code needs the room. Without bounds the call of traverse4_finish decides: 103 and
+// 112 registers and 2 blocks with spheres, 130 and one block for batches with interfaces (four such boxes
+// of 256^2 x 16 samples: 41.9 -> 39.8 ms).
 template <bool kSpheres, bool kMedia, bool kBatch = false, bool kWalls = false>
-__global__ void __launch_bounds__(256, (kSpheres || kMedia || kWalls) ? 1 : 4)
+__global__ void __launch_bounds__(256, (kMedia || kWalls) ? 2 : (kSpheres ? 3 : 4))
     k_shadow_any(DevScene s0, const DevScene *scenes, Paths P, Shadows S, int *counters) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
