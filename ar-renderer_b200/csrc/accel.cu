@@ -163,10 +163,13 @@ template <bool kAny, bool kWide, bool kTail> void launch_one(const DeviceAccel &
     PRB_CUDA(cudaGetLastError());
 }
 
-// Up to this many rays the launch's tail, 40 to 80 us with one lane a ray to the end, costs more than
-// the registers that the call of traverse4_finish takes from the loop (7 %). 1M-triangle soup, closest
-// hit, with / without, us: 4,096 rays 84 / 124, 262,144 209 / 241, 1.5M 505 / 526, 4.2M 1153 / 1122,
-// 16.8M 4187 / 3897.
+// Closest hits: up to this many rays the launch's tail, 35 to 60 us with one lane a ray to the end, costs
+// more than the registers that the call of traverse4_finish takes from the loop (5 %). us, one lane / tail
+// form: 1M-triangle soup, 4,096 rays 129 / 86, 262,144 250 / 210, 1.5M 543 / 510, 2.1M 676 / 648, 4.2M
+// 1137 / 1156, 16.8M 3971 / 4191; 100,003 triangles, 4.2M rays 1019 / 992, 8.4M 1813 / 1872; 4,096
+// triangles, 2.1M rays 445 / 438, 4.2M 769 / 789.
+// Any hits take the tail form at every size, as its loop spills nothing: 4,096 rays 111 / 57, 1.5M 420 / 354,
+// 4.2M 857 / 777, 16.8M 2791 / 2716; 4,096 triangles, 16.8M rays 1977 / 1949.
 constexpr int64_t kTailRays = 3 << 20;
 
 // wide: the 4-wide tree, each ray's hit a function of the ray and the tree alone; otherwise the binary
@@ -177,12 +180,12 @@ void launch_trace(const DeviceAccel &acc, const TraceArgs &q, bool anyHit, bool 
     if (!wide) {
         if (anyHit) launch_one<true, false, false>(acc, q);
         else launch_one<false, false, false>(acc, q);
+    } else if (anyHit) {
+        launch_one<true, true, true>(acc, q);
     } else if (q.n <= kTailRays) {
-        if (anyHit) launch_one<true, true, true>(acc, q);
-        else launch_one<false, true, true>(acc, q);
+        launch_one<false, true, true>(acc, q);
     } else {
-        if (anyHit) launch_one<true, true, false>(acc, q);
-        else launch_one<false, true, false>(acc, q);
+        launch_one<false, true, false>(acc, q);
     }
 }
 

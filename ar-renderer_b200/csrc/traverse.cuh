@@ -432,8 +432,6 @@ __device__ __forceinline__ void sort4(float &t0, int &r0, float &t1, int &r1, fl
     cswap(t1, r1, t2, r2);
 }
 
-// kSkipTransparent: primitives whose class byte (cls) has kTransparentBit do not count as hits;
-// intersecting one sets s.crossed.
 // The traversal stack as two per-thread arrays (local memory).
 struct LocalStack {
     int *ref;
@@ -487,11 +485,6 @@ struct HybridStack {
     __device__ __forceinline__ int node(int i) const { return i < kShort ? sh[i * kThreads].x : ref[i - kShort]; }
 };
 
-// kDeferUV (closest hit): a hit records only its leaf slot (s.hit.prim) and distance (s.tMax);
-// the caller repeats the winning primitive's test once at the end (finish_hit), which gives the
-// same t, u, v bit for bit. Fewer live registers in the loop let the slab planes be selected by
-// address as for any hit (ray-query benchmark, closest hit: 3,821 -> 3,926 Mrays/s; either change
-// alone was slower: 3,730 and 3,667).
 // Takes the next deferred child whose entry is still before tMax; false: the traversal is finished.
 template <class Stack> __device__ __forceinline__ bool traverse4_pop(TravState &s, Stack &stack) {
     while (s.sp > 0) {
@@ -505,6 +498,11 @@ template <class Stack> __device__ __forceinline__ bool traverse4_pop(TravState &
 }
 
 // One interior node (s.ref >= 0). Returns true when the ray's traversal is finished.
+// kDeferUV (closest hit): a hit records only its leaf slot (s.hit.prim) and distance (s.tMax);
+// the caller repeats the winning primitive's test once at the end (finish_hit), which gives the
+// same t, u, v bit for bit. Fewer live registers in the loop let the slab planes be selected by
+// address as for any hit (ray-query benchmark, closest hit: 3,821 -> 3,926 Mrays/s; either change
+// alone was slower: 3,730 and 3,667).
 template <bool kAny, bool kDeferUV, class Stack>
 __device__ __forceinline__ bool traverse4_node(const QNode *__restrict__ nodes, const TraceRay &r, TravState &s,
                                                Stack &stack, bool *overflow) {
@@ -571,6 +569,8 @@ __device__ __forceinline__ bool traverse4_node(const QNode *__restrict__ nodes, 
 }
 
 // One leaf (s.ref < 0). Returns true when the ray's traversal is finished.
+// kSkipTransparent: primitives whose class byte (cls) has kTransparentBit do not count as hits;
+// intersecting one sets s.crossed.
 template <bool kAny, bool kSpheres, bool kSkipTransparent, bool kDeferUV, class Stack>
 __device__ __forceinline__ bool traverse4_leaf(const LeafPrim *__restrict__ prims, const TraceRay &r, TravState &s,
                                                Stack &stack, const uint8_t *__restrict__ cls = nullptr) {
@@ -637,8 +637,8 @@ __device__ __forceinline__ Hit finish_hit(const LeafPrim *__restrict__ prims, co
 // lanes take entries off the rays' stacks (one entry per ray and step with more than four rays left, up
 // to eight with one), each lane tests one child box or one of a leaf's triangles, and what is hit goes
 // back on the stack, so a ray takes a step per level of the tree rather than per node. Measured (B200,
-// closest hit, us, one lane a ray to the end / this): 1,000 rays, 4,096 triangles 81 / 32; 4,096 rays,
-// 100,003 triangles 112 / 56; 1.5M rays, 100,003 triangles 450 / 421.
+// closest hit, us, one lane a ray to the end / this): 1,000 rays, 4,096 triangles 85 / 32; 4,096 rays,
+// 100,003 triangles 120 / 59; 1.5M rays, 100,003 triangles 457 / 421.
 //
 // The result is that of the one-lane walk bit for bit, so it does not depend on which rays a warp was left
 // with. Box and triangle arithmetic are those of the other traversals, and for a closest hit the walk's
@@ -660,7 +660,11 @@ __device__ __forceinline__ Hit finish_hit(const LeafPrim *__restrict__ prims, co
 // then still has room for such a walk, so a region cannot overflow.
 constexpr int kCoopRays = 8, kRayLanes = 4;
 constexpr int kLeafPad = kRayLanes - 1;  // records past the leaf array that the lanes of a group may load
-constexpr int kCoopBound = kStackSize - 24;  // trees with a larger bound are left to the one-lane traversal
+// Trees with a larger bound are left to the one-lane traversal. A ray is handed over with at most
+// kShortStack + 1 entries, and its region must hold the walk on top of them, which 47 would still do; 24
+// leave room to open two entries a step from the first step on. Trees between the two are not measured.
+constexpr int kCoopBound = kStackSize - 24;
+static_assert(kShortStack + 1 + kCoopBound <= kStackSize, "a ray's region holds what it brings and a walk");
 
 struct CoopState {
     TravState s;
@@ -929,9 +933,10 @@ __device__ __forceinline__ bool coop_ready(unsigned busy, bool active, int sp) {
 
 // A warp's step is either a node for the lanes at a node or a leaf for those at a leaf: with both in
 // every step, the leaf code ran with two or three lanes. Lanes at a leaf wait until kLeafLanes do, or
-// until no lane is at a node. Ray-query benchmark (2^24 rays, closest /
-// any hit, ms): both in every step 4.20 / 2.92; from 6 lanes 3.96 / 2.77, 8 lanes 3.90 / 2.74; 12 and 16
-// were 1 and 5 % slower than 8.
+// until no lane is at a node. From 1 / 4 / 8 / 12 lanes on: 2^24 rays, 1M triangles, closest 4.69 / 4.15 /
+// 3.97 / 3.97 ms, any hit 3.25 / 2.89 / 2.76 / 2.75; leaves of up to four of 100,003 triangles, 1.5M any-hit
+// rays 338 / 309 / 302 / 312 us, 200,003 closest 160 / 153 / 155 / 161; renders, ms: box 16.6 / 15.7 / 15.4 /
+// 15.5, fog 8.28 / 8.13 / 8.06 / 8.10, guided 8.25 / 8.13 / 8.05 / 8.11.
 constexpr int kLeafLanes = 8;
 __device__ __forceinline__ bool leaf_turn(unsigned busy, unsigned leaves) {
     return __popc(leaves) >= kLeafLanes || leaves == busy;

@@ -52,8 +52,13 @@ def _check(nodes, order, verts, rays, any_hit):
         return want
     np.testing.assert_array_equal(t.view(np.int32), want[1].view(np.int32))
     np.testing.assert_array_equal(prim >= 0, want[0] >= 0)
-    # Another primitive only where two lie at exactly the same distance.
-    assert (prim != want[0]).sum() <= max(1, n // 100000)
+    # Another primitive only where each of the two, alone, is hit at exactly that distance.
+    for k in np.flatnonzero(prim != want[0]):
+        for p in (prim[k], want[0][k]):
+            v = verts[p:p + 1]
+            one = _tree([(v.min((0, 1)), v.max((0, 1)), 0, 1)])
+            alone = trace.trace_rays(one, np.zeros(1, np.int32), v, rays[k:k + 1])
+            assert alone[0][0] == 0 and alone[1].view(np.int32)[0] == t.view(np.int32)[k]
     return want[0]
 
 
