@@ -645,8 +645,9 @@ __device__ __forceinline__ Hit finish_hit(const LeafPrim *__restrict__ prims, co
 // order is kept: an entry above another on a stack comes with all it leads to before it. Nodes may be
 // opened ahead of their turn (an entry is tested against tMax again when it is taken, and tMax only falls;
 // a child lies within its node's box and so is entered no earlier, see kLooseBound; the children are sorted by the one-lane walk's own network, in which entries that fall away later, being
-// farther than all that stay, do not change the order of the rest), but a leaf is tested only once all
-// entries above it are leaves that end in the same step. Of those the hits count in order: a leaf entered
+// farther than all that stay, do not change the order of the rest), and a leaf tested ahead of its turn is
+// done with if nothing in it is hit, but else waits until all entries above it are leaves that end in the
+// same step. Of those the hits count in order: a leaf entered
 // at or beyond an earlier leaf's hit is not visited (rounding can put a hit before its own box's entry, so
 // a later hit may be the nearer one and still not count), and equal distances go to the first. What the
 // order of one step cannot settle is handed back (true in its lane) for the one-lane traversal to start
@@ -757,9 +758,6 @@ __device__ __noinline__ CoopState traverse4_coop(const QNode *nodes, const LeafP
             entry = __int_as_float(v.y);
             work = entry < tMax;
         }
-        // Whether a leaf is tested in this step; if not it stays on the stack as it is.
-        bool inTurn = true;
-        if (!kAny && perRay > 1) inTurn = !(__ballot_sync(full, work && ref >= 0) & earlier);
         __syncwarp();
         float t = inf;   // entry distance of the child, or the leaf's own for its next four triangles
         int next = 0;
@@ -784,7 +782,7 @@ __device__ __noinline__ CoopState traverse4_coop(const QNode *nodes, const LeafP
                     t = box_entry(q, bx ? fx : nx, by ? fy : ny, bz ? fz : nz, bx ? nx : fx, by ? ny : fy, bz ? nz : fz,
                                   &te) && te < tMax ? te : inf;
                 }
-            } else if (inTurn) {
+            } else {
                 // Slots past the leaf's last belong to other leaves or are padding: loaded, not tested.
                 const LeafPrim *p = lp + ~ref + sub;
                 const float4 v0 = __ldg(&p->v0), v1 = __ldg(&p->v1), v2 = __ldg(&p->v2);
@@ -811,19 +809,23 @@ __device__ __noinline__ CoopState traverse4_coop(const QNode *nodes, const LeafP
             }
         }
         __syncwarp();
-        if (!kAny && perRay > 1) {
-            // A leaf behind one that goes on was tested too early.
-            if (__ballot_sync(full, goesOn) & earlier) inTurn = false;
-            if (work && ref < 0 && !inTurn) {
-                hit = nan = false;
-                t = sub == 0 ? entry : inf;
-                next = ref;
-            }
-        }
         const int myFirst = __popc(rays & ((1u << lane) - 1u)) * kRayLanes * perRay;  // of the ray this lane owns
         const bool own = (rays >> lane) & 1u;
         const unsigned ownLanes = own ? (perRay == 8 ? full : (1u << (kRayLanes * perRay)) - 1u) << myFirst : 0u;
-        const unsigned hits = __ballot_sync(full, hit);
+        unsigned hits = __ballot_sync(full, hit);
+        bool inTurn = true;
+        if (!kAny && perRay > 1) {
+            // A leaf below a node, or below one that goes on, with a hit in it: back as it is; without: done,
+            // or its next four triangles under the leaf's own entry.
+            inTurn = !(__ballot_sync(full, work && (ref >= 0 || goesOn)) & earlier);
+            if (work && ref < 0 && !inTurn) {
+                const bool again = (hits >> quad) & 0xfu;
+                hit = nan = false;
+                t = (again || goesOn) && sub == 0 ? entry : inf;
+                if (again) next = ref;
+            }
+            if (hits) hits = __ballot_sync(full, hit);
+        }
         if (hits) {
             if (!kAny) {
                 // The least distance of each group, of the groups up to it, and of the ray's.
