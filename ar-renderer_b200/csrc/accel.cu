@@ -165,9 +165,9 @@ template <bool kAny, bool kWide, bool kTail> void launch_one(const DeviceAccel &
 
 // Closest hits: up to this many rays the launch's tail, 35 to 60 us with one lane a ray to the end, costs
 // more than the registers that the call of traverse4_finish takes from the loop (5 %). us, one lane / tail
-// form: 1M-triangle soup, 4,096 rays 129 / 86, 262,144 250 / 210, 1.5M 543 / 510, 2.1M 676 / 648, 4.2M
-// 1137 / 1156, 16.8M 3971 / 4191; 100,003 triangles, 4.2M rays 1019 / 992, 8.4M 1813 / 1872; 4,096
-// triangles, 2.1M rays 445 / 438, 4.2M 769 / 789.
+// form: 1M-triangle soup, 4,096 rays 129 / 84, 262,144 254 / 205, 1.5M 557 / 504, 2.1M 665 / 650, 4.2M
+// 1142 / 1155, 16.8M 3987 / 4207; 100,003 triangles, 4.2M rays 1012 / 991, 8.4M 1812 / 1868; 4,096
+// triangles, 2.1M rays 441 / 432, 4.2M 775 / 787.
 // Any hits take the tail form at every size, as its loop spills nothing: 4,096 rays 111 / 57, 1.5M 420 / 354,
 // 4.2M 857 / 777, 16.8M 2791 / 2716; 4,096 triangles, 16.8M rays 1977 / 1949.
 constexpr int64_t kTailRays = 3 << 20;

@@ -638,7 +638,7 @@ __device__ __forceinline__ Hit finish_hit(const LeafPrim *__restrict__ prims, co
 // to eight with one), each lane tests one child box or one of a leaf's triangles, and what is hit goes
 // back on the stack, so a ray takes a step per level of the tree rather than per node. Measured (B200,
 // closest hit, us, one lane a ray to the end / this): 1,000 rays, 4,096 triangles 85 / 32; 4,096 rays,
-// 100,003 triangles 120 / 59; 1.5M rays, 100,003 triangles 457 / 421.
+// 100,003 triangles 119 / 57; 1.5M rays, 100,003 triangles 456 / 421.
 //
 // The result is that of the one-lane walk bit for bit, so it does not depend on which rays a warp was left
 // with. Box and triangle arithmetic are those of the other traversals, and for a closest hit the walk's
